@@ -2,7 +2,8 @@
 
 ``build_kernels()``  nvcc (sm_100a) -> ``eddl_b200/lib/libeddl_b200.so``: the CUDA kernels and
                      the C ABI declared in ``include/eddl_b200.h``.  Needs nothing but the
-                     CUDA toolkit and NCCL.
+                     CUDA toolkit and NCCL.  With it ``lib/_fastcall.so``, the binding's native caller
+                     (``host/fastcall.c``; skipped where Python's headers are missing).
 ``build_dropin()``   g++ -> ``baseline/_ref/libeddl_b200_dropin.so``: the C++ shim that defines
                      EDDL's ``gpu_*`` functions on top of the C ABI (``eddl_b200/shim``), the
                      distributed entry points and the net harness, linked with EDDL's own host
@@ -13,6 +14,7 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -60,6 +62,49 @@ def build_kernels(verbose=False):
         cmd = [NVCC, "-shared", "-o", lib] + objs + ["-gencode", "arch=compute_100a,code=sm_100a",
                                                      "-lnccl", "-lcuda", "-Xlinker", "-rpath,$ORIGIN"]
         subprocess.run(cmd, check=True)
+    build_fastcall(lib)
+    return lib
+
+
+def _fastcall_table():
+    """The C wrappers of fastcall.c, one per function that the header declares (see there)."""
+    sys.path.insert(0, ROOT)
+    from eddl_b200 import capi
+    out, rows = [], []
+    for name, ret, params in capi.declared_functions():
+        if ret != "int":
+            continue
+        short = name[len("eddlb200_"):]
+        decl, conv, args = [], [], []
+        for i, p in enumerate(params):
+            if "*" in p:
+                decl.append("void *p%d;" % i); conv.append("to_ptr(a[%d], &p%d)" % (i, i)); args.append("(void *)p%d" % i)
+            else:
+                base = p.replace("const", " ").split()[0]
+                kind = {"int": "int", "size_t": "size", "float": "float"}[base]
+                decl.append("%s p%d;" % (base, i)); conv.append("to_%s(a[%d], &p%d)" % (kind, i, i)); args.append("p%d" % i)
+        cond = " && ".join(["n == %d" % len(params)] + conv)
+        out.append("static int w_%s(PyObject *const *a, Py_ssize_t n, int *status) {\n    (void)a; %s\n    if (!(%s)) return 0;\n"
+                   "    Py_BEGIN_ALLOW_THREADS\n    *status = %s(%s);\n    Py_END_ALLOW_THREADS\n    return 1;\n}\n"
+                   % (short, " ".join(decl), cond, name, ", ".join(args)))
+        rows.append('    {"%s", w_%s},\n' % (short, short))
+    return ("".join(out) + "static const struct { const char *name; Wrapper fn; } g_table[] = {\n" + "".join(rows) + "    {NULL, NULL}};\n")
+
+
+def build_fastcall(kernels):
+    """gcc -> eddl_b200/lib/_fastcall.so, the native caller that the Python binding uses where it exists."""
+    inc = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        return None
+    src, table = os.path.join(PKG, "host", "fastcall.c"), os.path.join(LIBDIR, "obj", "fastcall_table.inc")
+    text = _fastcall_table()
+    if not os.path.exists(table) or open(table).read() != text:
+        open(table, "w").write(text)
+    lib = os.path.join(LIBDIR, "_fastcall.so")
+    if _newer(lib, [src, table, kernels]):
+        subprocess.run(["gcc", "-O2", "-fPIC", "-shared", "-Wno-incompatible-pointer-types", "-Wno-discarded-qualifiers", "-I" + inc,
+                        "-I" + os.path.join(ROOT, "include"), "-I" + os.path.dirname(table), src, "-o", lib,
+                        "-L" + LIBDIR, "-leddl_b200", "-Wl,-rpath,$ORIGIN"], check=True)
     return lib
 
 

@@ -5,6 +5,8 @@ declarations.  Loading fails loudly when the CUDA library has not been built: th
 fallback behind this module.
 """
 import ctypes
+import functools
+import importlib.util
 import os
 import re
 
@@ -42,6 +44,20 @@ class Error(RuntimeError):
     pass
 
 
+def _native_caller():
+    """The C caller built beside the library (host/fastcall.c), or None: ctypes then converts every argument."""
+    path = os.path.join(PKG, "lib", "_fastcall.so")
+    if not os.path.exists(path):
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location("_fastcall", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except ImportError:                   # built for another interpreter
+        return None
+
+
 class Lib:
     """The loaded C ABI.  ``lib.call('conv2d_fwd', dev, ...)`` raises Error on a non-zero status."""
 
@@ -56,6 +72,10 @@ class Lib:
             f.restype = ctypes.c_char_p if "char" in ret else ctypes.c_int
             f.argtypes = [_ctype(p) for p in params]
             self.fn[name[len("eddlb200_"):]] = f
+        native = _native_caller() if path == LIBPATH else None
+        if native is not None:
+            native.setup(DeviceArray, ctypes.Array, functools.partial(Lib.call, self), self._fail)
+            self.call = native.call       # same arguments, same errors, without ctypes on the way
 
     def last_error(self):
         return self.fn["last_error"]().decode()
@@ -64,7 +84,10 @@ class Lib:
         conv = [a.ptr if isinstance(a, DeviceArray) else a for a in args]
         st = self.fn[name](*conv)
         if st != 0:
-            raise Error("eddlb200_%s -> %d: %s" % (name, st, self.last_error()))
+            self._fail(name, st)
+
+    def _fail(self, name, st):
+        raise Error("eddlb200_%s -> %d: %s" % (name, st, self.last_error()))
 
     def device_count(self):
         n = ctypes.c_int(0)
@@ -105,7 +128,7 @@ class DeviceArray:
         self.size = int(np.prod(self.shape)) if len(self.shape) else 1
         p = ctypes.c_void_p()
         lib.call("alloc", dev, max(self.size, 1) * 4, ctypes.byref(p))
-        self.ptr = p
+        self.ptr, self.addr = p, p.value
 
     def numpy(self):
         out = np.empty(self.shape, dtype=np.float32)
@@ -117,7 +140,7 @@ class DeviceArray:
         try:
             if self.ptr:
                 self.lib.fn["free"](self.dev, self.ptr)
-                self.ptr = None
+                self.ptr = self.addr = None
         except Exception:
             pass
 
