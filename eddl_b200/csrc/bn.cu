@@ -45,6 +45,7 @@ __device__ __forceinline__ size_t item_offset(unsigned t, unsigned rc, unsigned 
 template <int MODE, bool VEC>
 __global__ void __launch_bounds__(kBlock) bn_stats_kernel(const float *__restrict__ x, const float *__restrict__ o,
                                                           float2 *__restrict__ partial, unsigned b, unsigned z, unsigned rc) {
+    EB_GRID_WAIT();
     __shared__ float sm[32];
     const unsigned j = blockIdx.x, s = blockIdx.y, nsplit = gridDim.y;
     const Slice sl = slice_of(b * rc, nsplit, s);
@@ -104,6 +105,7 @@ __global__ void __launch_bounds__(kBlock) bn_fwd_apply_kernel(const float *__res
                                                               const float *__restrict__ g, const float *__restrict__ beta,
                                                               float *mean_out, float *var_out,
                                                               unsigned b, unsigned z, unsigned rc, float eps, float momentum) {
+    EB_GRID_WAIT();
     __shared__ float sh[2];
     // slices in reverse launch order: the statistics pass finished with the highest slices, so those are what the L2 holds
     const unsigned j = blockIdx.x, nsplit = gridDim.y, s = nsplit - 1 - blockIdx.y;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kBlock) bn_bwd_apply_kernel(float *__restrict_
                                                               float *gbn_g, float *gbn_b, const float *__restrict__ bn_g,
                                                               const float *__restrict__ variance, float *mean1, float *mean2,
                                                               unsigned b, unsigned z, unsigned rc) {
+    EB_GRID_WAIT();
     __shared__ float sh[2];
     const unsigned j = blockIdx.x, nsplit = gridDim.y, s = nsplit - 1 - blockIdx.y;     // reverse launch order, see forward
     float s1, s2;
@@ -282,14 +285,14 @@ int eddlb200_bn_fwd(int dev, int b, int z, int rc, const float *input, float *ou
     if (trmode) {
         partial = (float2 *)scratch(cx, (size_t)z * S * sizeof(float2));
         if (!partial) return cudaErrorMemoryAllocation;
-        if (vec) bn_stats_kernel<0, true><<<grid, kBlock, 0, st>>>(input, nullptr, partial, b, z, rc);
-        else bn_stats_kernel<0, false><<<grid, kBlock, 0, st>>>(input, nullptr, partial, b, z, rc);
+        if (vec) eb::launch(bn_stats_kernel<0, true>, grid, kBlock, 0, st, input, nullptr, partial, b, z, rc);
+        else eb::launch(bn_stats_kernel<0, false>, grid, kBlock, 0, st, input, nullptr, partial, b, z, rc);
         EB_LAUNCH_CHECK("gpu_batchnorm_forward(stats)");
-        if (vec) bn_fwd_apply_kernel<true, true><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
-        else bn_fwd_apply_kernel<true, false><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        if (vec) eb::launch(bn_fwd_apply_kernel<true, true>, grid, kBlock, 0, st, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        else eb::launch(bn_fwd_apply_kernel<true, false>, grid, kBlock, 0, st, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
     } else {
-        if (vec) bn_fwd_apply_kernel<false, true><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
-        else bn_fwd_apply_kernel<false, false><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        if (vec) eb::launch(bn_fwd_apply_kernel<false, true>, grid, kBlock, 0, st, input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        else eb::launch(bn_fwd_apply_kernel<false, false>, grid, kBlock, 0, st, input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
     }
     EB_LAUNCH_CHECK("gpu_batchnorm_forward(apply)");
     return 0;
@@ -319,13 +322,13 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
     dim3 grid(z, S);
     float2 *partial = (float2 *)scratch(cx, (size_t)z * S * sizeof(float2));
     if (!partial) return cudaErrorMemoryAllocation;
-    if (vec) bn_stats_kernel<1, true><<<grid, kBlock, 0, st>>>(delta, opa, partial, b, z, rc);
-    else bn_stats_kernel<1, false><<<grid, kBlock, 0, st>>>(delta, opa, partial, b, z, rc);
+    if (vec) eb::launch(bn_stats_kernel<1, true>, grid, kBlock, 0, st, delta, opa, partial, b, z, rc);
+    else eb::launch(bn_stats_kernel<1, false>, grid, kBlock, 0, st, delta, opa, partial, b, z, rc);
     EB_LAUNCH_CHECK("gpu_batchnorm_backward(stats)");
-    if (vec && pd_zero) bn_bwd_apply_kernel<true, true><<<grid, kBlock, 0, st>>>(delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
-    else if (vec) bn_bwd_apply_kernel<true, false><<<grid, kBlock, 0, st>>>(delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
-    else if (pd_zero) bn_bwd_apply_kernel<false, true><<<grid, kBlock, 0, st>>>(delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
-    else bn_bwd_apply_kernel<false, false><<<grid, kBlock, 0, st>>>(delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
+    if (vec && pd_zero) eb::launch(bn_bwd_apply_kernel<true, true>, grid, kBlock, 0, st, delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
+    else if (vec) eb::launch(bn_bwd_apply_kernel<true, false>, grid, kBlock, 0, st, delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
+    else if (pd_zero) eb::launch(bn_bwd_apply_kernel<false, true>, grid, kBlock, 0, st, delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
+    else eb::launch(bn_bwd_apply_kernel<false, false>, grid, kBlock, 0, st, delta, opa, pdelta, partial, gbn_g, gbn_b, bn_g, variance, mean1, mean2, b, z, rc);
     EB_LAUNCH_CHECK("gpu_batchnorm_backward(apply)");
     return 0;
 }
@@ -418,14 +421,14 @@ extern "C" int eddlb200_bn_fwd_noalloc(int dev, int b, int z, int rc, const floa
     const bool vec = (rc % 4 == 0) && aligned16(input) && aligned16(output) && (!opa || aligned16(opa)) && (!relu_out || aligned16(relu_out));
     dim3 grid(z, S);
     if (trmode) {
-        if (vec) bn_stats_kernel<0, true><<<grid, kBlock, 0, st>>>(input, nullptr, partial, b, z, rc);
-        else bn_stats_kernel<0, false><<<grid, kBlock, 0, st>>>(input, nullptr, partial, b, z, rc);
+        if (vec) eb::launch(bn_stats_kernel<0, true>, grid, kBlock, 0, st, input, nullptr, partial, b, z, rc);
+        else eb::launch(bn_stats_kernel<0, false>, grid, kBlock, 0, st, input, nullptr, partial, b, z, rc);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "bn_fwd_noalloc(stats)");
-        if (vec) bn_fwd_apply_kernel<true, true><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
-        else bn_fwd_apply_kernel<true, false><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        if (vec) eb::launch(bn_fwd_apply_kernel<true, true>, grid, kBlock, 0, st, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        else eb::launch(bn_fwd_apply_kernel<true, false>, grid, kBlock, 0, st, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
     } else {
-        if (vec) bn_fwd_apply_kernel<false, true><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
-        else bn_fwd_apply_kernel<false, false><<<grid, kBlock, 0, st>>>(input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        if (vec) eb::launch(bn_fwd_apply_kernel<false, true>, grid, kBlock, 0, st, input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
+        else eb::launch(bn_fwd_apply_kernel<false, false>, grid, kBlock, 0, st, input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, b, z, rc, epsilon, momentum);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "bn_fwd_noalloc(apply)");
     return 0;

@@ -12,6 +12,7 @@ namespace {
 using namespace eb;
 
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ part, float *__restrict__ out, size_t count, int splits) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
         float s = 0.f;
@@ -22,6 +23,7 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restr
 
 // gbias[k] += sum_{n,p,q} dy[n,k,p,q]   (cpu_conv2D_grad, src/hardware/cpu/nn/cpu_conv.cpp:466-478)
 __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict__ dy, float *__restrict__ gbias, int n, int k, int pq) {
+    EB_GRID_WAIT();
     __shared__ float sm[32];
     const int kk = blockIdx.x;
     float s = 0.f;
@@ -41,6 +43,7 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const float *__restrict_
 // dst plane: rows of `ow` elements of which the first `vw` come from the source (the rest are zero), npix elements in all
 __global__ void __launch_bounds__(256) plane_gather_kernel(const float *__restrict__ src, float *__restrict__ dst, unsigned total,
                                                            int ihw, int iw, int sr, int sc, int ow, int vw, int npix, int pitch) {
+    EB_GRID_WAIT();
     const unsigned stride = gridDim.x * blockDim.x;
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
         const unsigned plane = idx / (unsigned)pitch, p = idx - plane * pitch;
@@ -56,6 +59,7 @@ __global__ void __launch_bounds__(256) plane_gather_kernel(const float *__restri
 // dx (full resolution) += the dense result at the pixels the convolution read; the others are left alone
 __global__ void __launch_bounds__(256) plane_scatter_add_kernel(const float *__restrict__ dense, float *__restrict__ dst, unsigned total,
                                                                 int ihw, int iw, int sr, int sc, int ow, int npix, int pitch) {
+    EB_GRID_WAIT();
     const unsigned stride = gridDim.x * blockDim.x;
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
         const unsigned plane = idx / (unsigned)pitch, p = idx - plane * pitch;
@@ -71,6 +75,7 @@ __global__ void __launch_bounds__(256) plane_scatter_add_kernel(const float *__r
 template <int V>
 __global__ void __launch_bounds__(256) plane_scatter_store_kernel(const float *__restrict__ dense, float *__restrict__ dst, unsigned total_v,
                                                                   int ihw, int iw, int sr, int sc, int oh, int ow, int pitch) {
+    EB_GRID_WAIT();
     const unsigned stride = gridDim.x * blockDim.x, ihw_v = ihw / V, iw_v = iw / V;
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total_v; idx += stride) {
         const unsigned plane = idx / ihw_v, r = idx - plane * ihw_v, y = r / iw_v, x0 = (r - y * iw_v) * V, oy = y / (unsigned)sr;
@@ -130,7 +135,7 @@ float *dense_buf(cudaStream_t st, int slot, size_t bytes) {
 int gather_planes(DevCtx *cx, cudaStream_t st, const float *src, float *dst, size_t planes, int ih, int iw, int sr, int sc, int oh, int ow, int pitch,
                   int valid_w = -1) {
     const unsigned total = (unsigned)(planes * pitch);
-    plane_gather_kernel<<<grid_for(total, 256), 256, 0, st>>>(src, dst, total, ih * iw, iw, sr, sc, ow, valid_w < 0 ? ow : valid_w, oh * ow, pitch);
+    eb::launch(plane_gather_kernel, grid_for(total, 256), 256, 0, st, src, dst, total, ih * iw, iw, sr, sc, ow, valid_w < 0 ? ow : valid_w, oh * ow, pitch);
     EB_LAUNCH_CHECK("conv2D(gather)");
     return 0;
 }
@@ -158,7 +163,7 @@ bool tc_enabled() {
 namespace eb {
 bool conv_tc_allowed() { return tc_enabled(); }
 int splitk_reduce_accumulate(DevCtx *cx, cudaStream_t st, const float *part, float *out, size_t count, int splits) {
-    splitk_reduce_kernel<<<grid_for(count, 256), 256, 0, st>>>(part, out, count, splits);
+    eb::launch(splitk_reduce_kernel, grid_for(count, 256), 256, 0, st, part, out, count, splits);
     EB_LAUNCH_CHECK("splitk_reduce");
     return 0;
 }
@@ -237,10 +242,10 @@ int eddlb200_conv2d_bwd_data(int dev, const float *dy, const float *w, float *dx
             int r = conv_tc_bwd_data(cx, st, d.g, dy, w, dense, precision, true);       // stores every element of the dense dx
             if (r == 0) {
                 const unsigned dense_elems = (unsigned)((size_t)n * c * d.pitch);
-                if (!dx_zero) plane_scatter_add_kernel<<<grid_for(dense_elems, 256), 256, 0, st>>>(dense, dx, dense_elems, ih * iw, iw, sr, sc, ow, oh * ow, d.pitch);
+                if (!dx_zero) eb::launch(plane_scatter_add_kernel, grid_for(dense_elems, 256), 256, 0, st, dense, dx, dense_elems, ih * iw, iw, sr, sc, ow, oh * ow, d.pitch);
                 else if (iw % 4 == 0 && ((uintptr_t)dx & 15) == 0)
-                    plane_scatter_store_kernel<4><<<grid_for(dx_elems / 4, 256), 256, 0, st>>>(dense, dx, (unsigned)(dx_elems / 4), ih * iw, iw, sr, sc, oh, ow, d.pitch);
-                else plane_scatter_store_kernel<1><<<grid_for(dx_elems, 256), 256, 0, st>>>(dense, dx, (unsigned)dx_elems, ih * iw, iw, sr, sc, oh, ow, d.pitch);
+                    eb::launch(plane_scatter_store_kernel<4>, grid_for(dx_elems / 4, 256), 256, 0, st, dense, dx, (unsigned)(dx_elems / 4), ih * iw, iw, sr, sc, oh, ow, d.pitch);
+                else eb::launch(plane_scatter_store_kernel<1>, grid_for(dx_elems, 256), 256, 0, st, dense, dx, (unsigned)dx_elems, ih * iw, iw, sr, sc, oh, ow, d.pitch);
                 EB_LAUNCH_CHECK("gpu_conv2D_back(scatter)");
                 g_conv_calls[dev][0]++;
                 return 0;
@@ -271,7 +276,7 @@ int eddlb200_conv2d_bwd_weight(int dev, const float *x, const float *dy, float *
     if (lz_any(cx)) { int status = 0; gw_zero = lz_take(cx, st, gw, gw_elems * sizeof(float), &status); if (status) return status; }
     ProfScope prof(cx, PROF_CONV_BWD_WEIGHT, 2.0 * n * (double)k * c * kr * kc * oh * ow);
     if (gbias) {
-        bias_grad_kernel<<<k, 256, 0, st>>>(dy, gbias, n, k, oh * ow);
+        eb::launch(bias_grad_kernel, k, 256, 0, st, dy, gbias, n, k, oh * ow);
         EB_LAUNCH_CHECK("gpu_conv2D_grad(bias)");
     }
     if (tc_enabled() && g_conv_dense && kr == 3 && kc == 3 && sr == 1 && sc == 1 && pad_top == 1 && pad_left == 1 && ih == oh && iw == ow &&

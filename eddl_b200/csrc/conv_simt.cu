@@ -111,6 +111,7 @@ struct PartialEpi {   // split-K partial: part[z][m][j]
 
 template <typename Ops, typename Epi>
 __global__ void __launch_bounds__(TB) igemm_simt_kernel(Ops ops, Epi epi, int k_per_split) {
+    EB_GRID_WAIT();
     __shared__ float As[BK][BM + 4];
     __shared__ float Bs[BK][BN + 4];
     const int M = ops.M(), N = ops.N(), K = ops.K();
@@ -170,7 +171,7 @@ int conv_simt_fwd(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x
     FwdEpi epi{g, y, bias};
     const long long N = (long long)g.n * g.oh * g.ow;
     dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(g.k, BM), 1);
-    igemm_simt_kernel<<<grid, TB, 0, st>>>(ops, epi, g.c * g.kr * g.kc);
+    eb::launch(igemm_simt_kernel<FwdOps, FwdEpi>, grid, TB, 0, st, ops, epi, g.c * g.kr * g.kc);
     EB_LAUNCH_CHECK("gpu_conv2D");
     return 0;
 }
@@ -180,7 +181,7 @@ int conv_simt_bwd_data(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const flo
     BwdDataEpi epi{g, dx};
     const long long N = (long long)g.n * g.ih * g.iw;
     dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(g.c, BM), 1);
-    igemm_simt_kernel<<<grid, TB, 0, st>>>(ops, epi, g.k * g.kr * g.kc);
+    eb::launch(igemm_simt_kernel<BwdDataOps, BwdDataEpi>, grid, TB, 0, st, ops, epi, g.k * g.kr * g.kc);
     EB_LAUNCH_CHECK("gpu_conv2D_back");
     return 0;
 }
@@ -203,7 +204,7 @@ int conv_simt_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const f
     if (!part) return cudaErrorMemoryAllocation;
     PartialEpi epi{part, N, MN};
     dim3 grid((unsigned)ceil_div(N, BN), (unsigned)ceil_div(M, BM), splits);
-    igemm_simt_kernel<<<grid, TB, 0, st>>>(ops, epi, k_per_split);
+    eb::launch(igemm_simt_kernel<BwdWeightOps, PartialEpi>, grid, TB, 0, st, ops, epi, k_per_split);
     EB_LAUNCH_CHECK("gpu_conv2D_grad");
     return splitk_reduce_accumulate(cx, st, part, gw, MN, splits);
 }

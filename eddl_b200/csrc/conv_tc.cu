@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 8) tmem_alloc(smem_u32(tmem_slot), 512);
+    EB_GRID_WAIT();             // everything above overlaps the end of the kernel before this one
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1202,6 +1203,7 @@ struct TableArgs {
 };
 
 __global__ void __launch_bounds__(256) build_tables_kernel(TableArgs T) {
+    EB_GRID_WAIT();
     const ConvGeom g = T.g;
     const int pq = g.oh * g.ow, hw = g.ih * g.iw, rs = g.kr * g.kc;
     const long long total = (long long)T.M_total + T.K_pad + T.N_total;
@@ -1351,6 +1353,7 @@ __device__ __forceinline__ void pack_b_tile(const float *__restrict__ src, const
 
 __global__ void __launch_bounds__(256) pack_b_kernel(const float *__restrict__ src, const int *__restrict__ rowB, const int *__restrict__ kB,
                                                      float *__restrict__ packed, int bn, int n_total, int tiles_n, int row_fastest, int prec) {
+    EB_GRID_WAIT();
     __shared__ float tile[128][BK + 1];
     pack_b_tile(src, rowB, kB, packed, bn, n_total, tiles_n, row_fastest, prec, blockIdx.x, blockIdx.y, tile);
 }
@@ -1363,6 +1366,7 @@ constexpr int kMaxPackJobs = 256;
 struct MultiPackArgs { const PackJob *jobs; int n; unsigned short slot[kMaxPackJobs]; unsigned start[kMaxPackJobs + 1]; };
 
 __global__ void __launch_bounds__(256) pack_b_multi_kernel(const __grid_constant__ MultiPackArgs A) {
+    EB_GRID_WAIT();
     __shared__ float tile[128][BK + 1];
     // which job does this block belong to: the last one whose first block is <= blockIdx.x
     int lo = 0, hi = A.n - 1;
@@ -1383,7 +1387,7 @@ int launch_variant(DevCtx *cx, cudaStream_t st, const TcParams &P, dim3 grid, in
         if (e != cudaSuccess) return cuda_status(e, "conv_tc(smem attribute)");
         configured = true;
     }
-    igemm_tc_kernel<BN_, PREC, WGRAD, BGATHER, TMA><<<grid, threads_of(TMA), SMEM, st>>>(P);
+    eb::launch(igemm_tc_kernel<BN_, PREC, WGRAD, BGATHER, TMA>, grid, threads_of(TMA), SMEM, st, P);
     EB_LAUNCH_CHECK("conv_tc");
     return 0;
 }
@@ -1509,7 +1513,7 @@ const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::arr
         A.slot[A.n] = (unsigned short)i; A.start[A.n] = total; total += e.blocks; seen[i] = v; A.n++;
     }
     A.start[A.n] = total;
-    pack_b_multi_kernel<<<total, 256, 0, st>>>(A);
+    eb::launch(pack_b_multi_kernel, total, 256, 0, st, A);
     count_launch(cx);
     if (cudaGetLastError() != cudaSuccess) return nullptr;
     for (int i = 0; i < A.n; i++) pc.entries[A.slot[i]].version = seen[A.slot[i]];
@@ -1519,6 +1523,7 @@ const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::arr
 // out[i] = sum_s part[s][i] (+ bias[(i / plane) % nbias])      (split-K forward)
 __global__ void __launch_bounds__(256) splitk_store_kernel(const float *__restrict__ part, float *__restrict__ out, size_t count, int splits,
                                                            const float *__restrict__ bias, int plane, int nbias) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
         float v = 0.f;
@@ -1677,7 +1682,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     T.rowA = (int2 *)(tb + o_rowA); T.kA = (int2 *)(tb + o_kA); T.rowB = (int *)(tb + o_rowB); T.kB = (int *)(tb + o_kB); T.outM = (int *)(tb + o_outM); T.kC = (int *)(tb + o_kC);
     if (build) {
         const long long entries = (long long)T.M_total + T.K_pad + T.N_total;
-        build_tables_kernel<<<grid_for((size_t)entries, 256), 256, 0, st>>>(T);
+        eb::launch(build_tables_kernel, grid_for((size_t)entries, 256), 256, 0, st, T);
         EB_LAUNCH_CHECK("conv_tc(tables)");
     }
     P.packedB = nullptr;
@@ -1690,7 +1695,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
         if (!img) {
             // no cached image (tables not cached, cache full, or allocation failed): pack into the scratch arena for this call
             dim3 pgrid(kblocks, tiles_n);
-            pack_b_kernel<<<pgrid, 256, 0, st>>>(srcB, T.rowB, T.kB, (float *)(ws + o_pack), bn, T.N_total, tiles_n, b_row_fastest, precision);
+            eb::launch(pack_b_kernel, pgrid, 256, 0, st, srcB, T.rowB, T.kB, (float *)(ws + o_pack), bn, T.N_total, tiles_n, b_row_fastest, precision);
             EB_LAUNCH_CHECK("conv_tc(pack weights)");
             img = (const float *)(ws + o_pack);
         }
@@ -1727,7 +1732,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     if (splits > 1) {
         if (mode == 0 || out_zero || (mode == 4 && T.ca != 1)) {
             // `out` holds nothing to add to: store the sum of the partials (0 + p0 + p1 + ...)
-            splitk_store_kernel<<<grid_for(out_total, 256), 256, 0, st>>>((const float *)(ws + o_part), out, out_total, splits, mode == 0 ? bias : nullptr, g.oh * g.ow, g.k);
+            eb::launch(splitk_store_kernel, grid_for(out_total, 256), 256, 0, st, (const float *)(ws + o_part), out, out_total, splits, mode == 0 ? bias : nullptr, g.oh * g.ow, g.k);
             EB_LAUNCH_CHECK("conv_tc(split-K store)");
             return 0;
         }
@@ -1771,6 +1776,7 @@ int run(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, const
 // Gather-form col2im for the GEMM route of backward-data: dx[n,c,y,x] += sum over the taps (r,s) of the pixel's stride
 // residue class of T[n][(c,r,s)][p][q], p = (y+pt-r)/sr, q = (x+pl-s)/sc.  One thread per dx element, no atomics.
 __global__ void __launch_bounds__(256) col2im_gather_kernel(ConvGeom g, const float *__restrict__ T, float *__restrict__ dx) {
+    EB_GRID_WAIT();
     const int hw = g.ih * g.iw, pq = g.oh * g.ow, rs = g.kr * g.kc;
     const long long total = (long long)g.n * g.c * hw;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -1794,6 +1800,7 @@ __global__ void __launch_bounds__(256) col2im_gather_kernel(ConvGeom g, const fl
 
 // out[c][r] = in[r][c] for a small rows x cols matrix (the weight tensor of a few-channel layer)
 __global__ void __launch_bounds__(256) transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int rows, int cols) {
+    EB_GRID_WAIT();
     const size_t total = (size_t)rows * cols, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const int c = (int)(i / rows), r = (int)(i - (size_t)c * rows);
@@ -1830,7 +1837,7 @@ int run_small_c_bwd_data(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g
         else wcap[dev] = w_elems;
     }
     if (dense) {
-        transpose_kernel<<<grid_for(w_elems, 256), 256, 0, st>>>(w, wt[dev], g.k, g.c * rs);
+        eb::launch(transpose_kernel, grid_for(w_elems, 256), 256, 0, st, w, wt[dev], g.k, g.c * rs);
         EB_LAUNCH_CHECK("conv_tc(transpose weights)");
         if (watch_any(cx)) note_write(cx, wt[dev], w_elems * sizeof(float));       // the packed image of the copy is stale now
         // the plane as one row of pq pixels: a 1x1 layer does not care about its two-dimensional shape
@@ -1846,7 +1853,7 @@ int run_small_c_bwd_data(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g
         T.M_total = g.n * pq; T.N_total = g.c * rs; T.K_total = g.k; P.limY = 1; P.limX = 1; P.out_n_stride = pq;
         if (int r = run_one(cx, st, dev, T, P, dy, w, tbuf[dev], nullptr, precision, t_elems, false)) return r;
     }
-    col2im_gather_kernel<<<grid_for((size_t)g.n * g.c * g.ih * g.iw, 256), 256, 0, st>>>(g, tbuf[dev], dx);
+    eb::launch(col2im_gather_kernel, grid_for((size_t)g.n * g.c * g.ih * g.iw, 256), 256, 0, st, g, tbuf[dev], dx);
     EB_LAUNCH_CHECK("conv_tc(col2im gather)");
     return 0;
 }

@@ -18,6 +18,7 @@ constexpr int kBlock = 256;
 
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map1_kernel(const float *a, float *b, size_t n4, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t j = i; j < n4; j += stride) {
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(kBlock) map1_kernel(const float *a, float *b, 
 
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map1_scalar_kernel(const float *a, float *b, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) b[j] = f(a[j]);
 }
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(kBlock) map1_scalar_kernel(const float *a, flo
 // c = f(a, b, c)
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map3_kernel(const float *a, const float *b, float *c, size_t n4, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t j = i; j < n4; j += stride) {
@@ -51,6 +54,7 @@ __global__ void __launch_bounds__(kBlock) map3_kernel(const float *a, const floa
 
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map3_scalar_kernel(const float *a, const float *b, float *c, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) c[j] = f(a[j], b[j], F::reads_c ? c[j] : 0.f);
 }
@@ -58,6 +62,7 @@ __global__ void __launch_bounds__(kBlock) map3_scalar_kernel(const float *a, con
 // c = f(a, b); r = max(c, 0): a recorded sum together with the ReLU that follows it.  n4 = 0 runs everything in the scalar loop.
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map3_relu_kernel(const float *a, const float *b, float *c, float *r, size_t n4, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t j = i; j < n4; j += stride) {
@@ -75,6 +80,7 @@ __global__ void __launch_bounds__(kBlock) map3_relu_kernel(const float *a, const
 // b = c = f(a): one source copied into two destinations.  n4 = 0 runs everything in the scalar loop.
 template <typename F>
 __global__ void __launch_bounds__(kBlock) map1_twice_kernel(const float *a, float *b, float *c, size_t n4, size_t n, F f) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t j = i; j < n4; j += stride) {
@@ -97,9 +103,9 @@ int launch1(DevCtx *cx, cudaStream_t st, const float *a, float *b, size_t n, F f
     ProfScope prof(cx, PROF_ELEMENTWISE, bytes_per_element * n);
     if (aligned16(a) && aligned16(b)) {
         size_t n4 = n / 4;
-        map1_kernel<<<grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st>>>(a, b, n4, n, f);
+        eb::launch(map1_kernel<F>, grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st, a, b, n4, n, f);
     } else {
-        map1_scalar_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(a, b, n, f);
+        eb::launch(map1_scalar_kernel<F>, grid_for(n, kBlock), kBlock, 0, st, a, b, n, f);
     }
     EB_LAUNCH_CHECK(what);
     return 0;
@@ -115,9 +121,9 @@ int launch3(DevCtx *cx, cudaStream_t st, const float *a, const float *b, float *
     ProfScope prof(cx, PROF_ELEMENTWISE, (bytes_per_element > 0 ? bytes_per_element : (F::reads_c ? 16.0 : 12.0)) * n);
     if (aligned16(a) && aligned16(b) && aligned16(c)) {
         size_t n4 = n / 4;
-        map3_kernel<<<grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st>>>(a, b, c, n4, n, f);
+        eb::launch(map3_kernel<F>, grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st, a, b, c, n4, n, f);
     } else {
-        map3_scalar_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(a, b, c, n, f);
+        eb::launch(map3_scalar_kernel<F>, grid_for(n, kBlock), kBlock, 0, st, a, b, c, n, f);
     }
     EB_LAUNCH_CHECK(what);
     return 0;
@@ -189,6 +195,7 @@ struct CceDeltaF {
 // rows are not a multiple of four long).  32-bit index arithmetic: the entry points refuse tensors of 2^31 elements or more.
 template <bool BACK, int V>
 __global__ void __launch_bounds__(kBlock) pad_kernel(float *a, float *b, unsigned total_v, int h, int w, int top, int left, int bh, int bw) {
+    EB_GRID_WAIT();
     const unsigned stride = gridDim.x * blockDim.x, wv = (unsigned)w / V;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total_v; i += stride) {
         const unsigned t = i / wv, x = (i - t * wv) * V, plane = t / (unsigned)h, y = t - plane * h;
@@ -210,6 +217,7 @@ struct FillSeg { float *p; unsigned long long n; float v; unsigned pad; };
 struct FillChunk { unsigned seg; unsigned offset_k; };
 constexpr unsigned kFillChunk = 16384;
 __global__ void __launch_bounds__(kBlock) fill_multi_kernel(const FillSeg *__restrict__ segs, const FillChunk *__restrict__ chunks, int nchunks) {
+    EB_GRID_WAIT();
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const FillChunk ch = chunks[c];
         const FillSeg sg = segs[ch.seg];
@@ -240,7 +248,7 @@ int pend_copy_flush(DevCtx *cx, cudaStream_t st) {
         EB_READS(p.src, n * sizeof(float)); EB_WRITES(p.dst, n * sizeof(float)); EB_WRITES(p.dst2, n * sizeof(float));
         ProfScope prof(cx, PROF_ELEMENTWISE, 12.0 * n);             // one read, two writes (the two in-place adds it replaces move 24)
         const size_t n4 = (aligned16(p.src) && aligned16(p.dst) && aligned16(p.dst2)) ? n / 4 : 0;
-        map1_twice_kernel<<<grid_for(n4 ? n4 : n, kBlock), kBlock, 0, st>>>(p.src, p.dst, p.dst2, n4, n, AxpbZeroF{p.sa, p.sb});
+        eb::launch(map1_twice_kernel<AxpbZeroF>, grid_for(n4 ? n4 : n, kBlock), kBlock, 0, st, p.src, p.dst, p.dst2, n4, n, AxpbZeroF{p.sa, p.sb});
         EB_LAUNCH_CHECK("gpu_add (two destinations)");
         return 0;
     }
@@ -250,8 +258,8 @@ int pend_copy_flush(DevCtx *cx, cudaStream_t st) {
 int launch_zero_fill(DevCtx *cx, cudaStream_t st, float *p, size_t n) {
     if (n == 0) return 0;
     ProfScope prof(cx, PROF_ELEMENTWISE, 4.0 * n);
-    if (aligned16(p)) { const size_t n4 = n / 4; map1_kernel<<<grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st>>>(p, p, n4, n, FillF{0.f}); }
-    else map1_scalar_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(p, p, n, FillF{0.f});
+    if (aligned16(p)) { const size_t n4 = n / 4; eb::launch(map1_kernel<FillF>, grid_for(n4 ? n4 : 1, kBlock), kBlock, 0, st, p, p, n4, n, FillF{0.f}); }
+    else eb::launch(map1_scalar_kernel<FillF>, grid_for(n, kBlock), kBlock, 0, st, p, p, n, FillF{0.f});
     EB_LAUNCH_CHECK("gpu_fill_(deferred)");
     return 0;
 }
@@ -288,7 +296,7 @@ int eddlb200_fill_multi(int dev, float *const *ptrs, const size_t *sizes, const 
     ProfScope prof(cx, PROF_ELEMENTWISE, 4.0 * total);
     int blocks = (int)chunks.size();
     if (blocks > EDDLB200_NUM_SMS * 8) blocks = EDDLB200_NUM_SMS * 8;
-    fill_multi_kernel<<<blocks, kBlock, 0, st>>>((const FillSeg *)tab, (const FillChunk *)(tab + off_c), (int)chunks.size());
+    eb::launch(fill_multi_kernel, blocks, kBlock, 0, st, (const FillSeg *)tab, (const FillChunk *)(tab + off_c), (int)chunks.size());
     EB_LAUNCH_CHECK("gpu_fill_(batched)");
     return 0;
 }
@@ -314,7 +322,7 @@ int eddlb200_relu_fwd(int dev, const float *a, float *b, size_t n) {
             EB_WRITES(p.dst, n * sizeof(float)); EB_WRITES(b, n * sizeof(float));
             ProfScope prof(cx, PROF_ELEMENTWISE, 16.0 * n);          // two reads, two writes (the two adds and the ReLU it replaces move 28)
             const size_t n4 = (aligned16(p.src) && aligned16(p.src2) && aligned16(p.dst) && aligned16(b)) ? n / 4 : 0;
-            map3_relu_kernel<<<grid_for(n4 ? n4 : n, kBlock), kBlock, 0, st>>>(p.src, p.src2, p.dst, b, n4, n, Sum2IntoZeroF{p.sa, p.sb, p.s2, p.t2});
+            eb::launch(map3_relu_kernel<Sum2IntoZeroF>, grid_for(n4 ? n4 : n, kBlock), kBlock, 0, st, p.src, p.src2, p.dst, b, n4, n, Sum2IntoZeroF{p.sa, p.sb, p.s2, p.t2});
             EB_LAUNCH_CHECK("gpu_add + gpu_relu");
             return 0;
         }
@@ -410,9 +418,9 @@ int eddlb200_pad(int dev, const float *a, float *b, int n, int c, int h, int w, 
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * total);
     EB_REQUIRE(total < 0x7fffffffull, "gpu_pad: tensor larger than 2^31 elements");
     if (w % 4 == 0 && ((uintptr_t)a & 15) == 0)
-        pad_kernel<false, 4><<<grid_for(total / 4, kBlock), kBlock, 0, st>>>(const_cast<float *>(a), b, (unsigned)(total / 4), h, w, top, left, h + top + bottom, w + left + right);
+        eb::launch(pad_kernel<false, 4>, grid_for(total / 4, kBlock), kBlock, 0, st, const_cast<float *>(a), b, (unsigned)(total / 4), h, w, top, left, h + top + bottom, w + left + right);
     else
-        pad_kernel<false, 1><<<grid_for(total, kBlock), kBlock, 0, st>>>(const_cast<float *>(a), b, (unsigned)total, h, w, top, left, h + top + bottom, w + left + right);
+        eb::launch(pad_kernel<false, 1>, grid_for(total, kBlock), kBlock, 0, st, const_cast<float *>(a), b, (unsigned)total, h, w, top, left, h + top + bottom, w + left + right);
     EB_LAUNCH_CHECK("gpu_pad");
     return 0;
 }
@@ -426,9 +434,9 @@ int eddlb200_pad_bwd(int dev, float *a_delta, const float *b_delta, int n, int c
     ProfScope prof(cx, PROF_ELEMENTWISE, 12.0 * total);
     EB_REQUIRE(total < 0x7fffffffull, "gpu_pad_back: tensor larger than 2^31 elements");
     if (w % 4 == 0 && ((uintptr_t)a_delta & 15) == 0)
-        pad_kernel<true, 4><<<grid_for(total / 4, kBlock), kBlock, 0, st>>>(a_delta, const_cast<float *>(b_delta), (unsigned)(total / 4), h, w, top, left, h + top + bottom, w + left + right);
+        eb::launch(pad_kernel<true, 4>, grid_for(total / 4, kBlock), kBlock, 0, st, a_delta, const_cast<float *>(b_delta), (unsigned)(total / 4), h, w, top, left, h + top + bottom, w + left + right);
     else
-        pad_kernel<true, 1><<<grid_for(total, kBlock), kBlock, 0, st>>>(a_delta, const_cast<float *>(b_delta), (unsigned)total, h, w, top, left, h + top + bottom, w + left + right);
+        eb::launch(pad_kernel<true, 1>, grid_for(total, kBlock), kBlock, 0, st, a_delta, const_cast<float *>(b_delta), (unsigned)total, h, w, top, left, h + top + bottom, w + left + right);
     EB_LAUNCH_CHECK("gpu_pad_back");
     return 0;
 }

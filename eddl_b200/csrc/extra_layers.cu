@@ -20,6 +20,7 @@ constexpr int kBlock = 256;
 // dest[(j / src_stride) * steps + j % src_stride] = src[j]   (derivative: src[j] += dest[...])
 template <bool DERIV>
 __global__ void __launch_bounds__(kBlock) concat_kernel(float *__restrict__ dest, float *__restrict__ src, size_t n, unsigned src_stride, unsigned steps) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
         const size_t q = j / src_stride, k = j - q * src_stride;
@@ -30,6 +31,7 @@ __global__ void __launch_bounds__(kBlock) concat_kernel(float *__restrict__ dest
 
 // B[row_b][col_b] = A[row_b / sr][col_b / sc] over all (image, channel, row) rows at once
 __global__ void __launch_bounds__(kBlock) repeat_nn_kernel(const float *__restrict__ a, float *__restrict__ b, size_t nb, int bw, int aw, int sr, int sc) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += stride) {
         const size_t row_b = i / bw; const int col_b = (int)(i - row_b * bw);
@@ -40,6 +42,7 @@ __global__ void __launch_bounds__(kBlock) repeat_nn_kernel(const float *__restri
 // A[row_a][col_a] += D over its sr x sc block, added one by one in row-major order of the block (the order in which the
 // reference's loop over D meets them), without atomics: one thread per element of A
 __global__ void __launch_bounds__(kBlock) repeat_nn_bwd_kernel(const float *__restrict__ d, float *__restrict__ a, size_t na, int dw, int aw, int sr, int sc) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < na; i += stride) {
         const size_t row_a = i / aw; const int col_a = (int)(i - row_a * aw);
@@ -53,6 +56,7 @@ __global__ void __launch_bounds__(kBlock) repeat_nn_bwd_kernel(const float *__re
 // B[n,c,i,j] = apply[n] ? A[n,c,flip(i,j)] : A[n,c,i,j]
 __global__ void __launch_bounds__(kBlock) flip_kernel(const float *__restrict__ a, float *__restrict__ b, size_t total, int c, int h, int w, int axis,
                                                       const unsigned char *__restrict__ apply) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t plane = (size_t)h * w, image = plane * c;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -69,6 +73,7 @@ __global__ void __launch_bounds__(kBlock) flip_kernel(const float *__restrict__ 
 // B[n,c,i,j] = A[n,c, i*hc/BH + y0, j*wc/BW + x0] with (y0, x0, hc, wc) per image
 __global__ void __launch_bounds__(kBlock) crop_scale_kernel(const float *__restrict__ a, float *__restrict__ b, size_t total, int c, int ah, int aw, int bh, int bw,
                                                             const int4 *__restrict__ box) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t bplane = (size_t)bh * bw, bimage = bplane * c;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -92,6 +97,7 @@ __host__ __device__ __forceinline__ int scale_src(int b, int off, int n_new, int
     return a;
 }
 __global__ void __launch_bounds__(kBlock) scale_kernel(const float *__restrict__ a, float *__restrict__ b, size_t total, ScaleGeom g) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t bplane = (size_t)g.bh * g.bw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -107,6 +113,7 @@ __global__ void __launch_bounds__(kBlock) scale_kernel(const float *__restrict__
 // A[ai][aj] += every B[bi][bj] that maps to it, added one by one in row-major order of B (cpu_single_scale_back, :140-190),
 // one thread per element of A: the mapping is monotonic, so the candidates of a source row are the output rows around ai*scale.
 __global__ void __launch_bounds__(kBlock) scale_bwd_kernel(float *__restrict__ a, const float *__restrict__ b, size_t total, ScaleGeom g) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t aplane = (size_t)g.ah * g.aw;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -137,6 +144,7 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
     return (float)(z >> 40) * (1.0f / 16777216.0f);       // 24 random bits -> [0, 1)
 }
 __global__ void __launch_bounds__(kBlock) rand_binary_kernel(float *__restrict__ a, size_t n, float p, unsigned long long seed, unsigned long long offset) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) a[i] = uniform01(seed, offset + i) < p ? 1.0f : 0.0f;
 }
@@ -158,8 +166,8 @@ int eddlb200_concat(int dev, float *a, float *const *parts, const size_t *part_s
     for (int i = 0; i < nparts; i++) {
         const size_t n = part_sizes[i];
         if (n) {
-            if (derivative) { EB_MODIFIES(parts[i], n * sizeof(float)); concat_kernel<true><<<grid_for(n, kBlock), kBlock, 0, st>>>(a + offset, parts[i], n, (unsigned)part_strides[i], (unsigned)steps); }
-            else { EB_READS(parts[i], n * sizeof(float)); concat_kernel<false><<<grid_for(n, kBlock), kBlock, 0, st>>>(a + offset, parts[i], n, (unsigned)part_strides[i], (unsigned)steps); }
+            if (derivative) { EB_MODIFIES(parts[i], n * sizeof(float)); eb::launch(concat_kernel<true>, grid_for(n, kBlock), kBlock, 0, st, a + offset, parts[i], n, (unsigned)part_strides[i], (unsigned)steps); }
+            else { EB_READS(parts[i], n * sizeof(float)); eb::launch(concat_kernel<false>, grid_for(n, kBlock), kBlock, 0, st, a + offset, parts[i], n, (unsigned)part_strides[i], (unsigned)steps); }
             EB_LAUNCH_CHECK("gpu_concat");
         }
         offset += part_strides[i];
@@ -174,7 +182,7 @@ int eddlb200_repeat_nn(int dev, const float *a, float *b, size_t rows_a, int col
     if (!nb) return 0;
     EB_READS(a, rows_a * cols_a * sizeof(float)); EB_WRITES(b, nb * sizeof(float));
     ProfScope prof(cx, PROF_ELEMENTWISE, 4.0 * rows_a * cols_a + 4.0 * nb);
-    repeat_nn_kernel<<<grid_for(nb, kBlock), kBlock, 0, st>>>(a, b, nb, cols_a * size_c, cols_a, size_r, size_c);
+    eb::launch(repeat_nn_kernel, grid_for(nb, kBlock), kBlock, 0, st, a, b, nb, cols_a * size_c, cols_a, size_r, size_c);
     EB_LAUNCH_CHECK("gpu_repeat_nn");
     return 0;
 }
@@ -186,7 +194,7 @@ int eddlb200_repeat_nn_bwd(int dev, const float *d, float *a, size_t rows_a, int
     if (!na) return 0;
     EB_READS(d, na * size_r * size_c * sizeof(float)); EB_MODIFIES(a, na * sizeof(float));
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * na + 4.0 * na * size_r * size_c);
-    repeat_nn_bwd_kernel<<<grid_for(na, kBlock), kBlock, 0, st>>>(d, a, na, cols_a * size_c, cols_a, size_r, size_c);
+    eb::launch(repeat_nn_bwd_kernel, grid_for(na, kBlock), kBlock, 0, st, d, a, na, cols_a * size_c, cols_a, size_r, size_c);
     EB_LAUNCH_CHECK("gpu_d_repeat_nn");
     return 0;
 }
@@ -202,7 +210,7 @@ int eddlb200_flip_batch(int dev, const float *a, float *b, int n, int c, int h, 
     cudaError_t e = cudaMemcpyAsync(flags, apply_host, (size_t)n, cudaMemcpyHostToDevice, st);      // pageable source: staged before return
     if (e != cudaSuccess) return cuda_status(e, "gpu_flip_random(flags)");
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * total);
-    flip_kernel<<<grid_for(total, kBlock), kBlock, 0, st>>>(a, b, total, c, h, w, axis, flags);
+    eb::launch(flip_kernel, grid_for(total, kBlock), kBlock, 0, st, a, b, total, c, h, w, axis, flags);
     EB_LAUNCH_CHECK("gpu_flip_random");
     return 0;
 }
@@ -225,7 +233,7 @@ int eddlb200_crop_scale_batch(int dev, const float *a, float *b, int n, int c, i
     cudaError_t e = cudaMemcpyAsync(dbox, box.data(), (size_t)n * sizeof(int4), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_status(e, "gpu_crop_scale_random(boxes)");
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * total);
-    crop_scale_kernel<<<grid_for(total, kBlock), kBlock, 0, st>>>(a, b, total, c, ah, aw, bh, bw, dbox);
+    eb::launch(crop_scale_kernel, grid_for(total, kBlock), kBlock, 0, st, a, b, total, c, ah, aw, bh, bw, dbox);
     EB_LAUNCH_CHECK("gpu_crop_scale_random");
     return 0;
 }
@@ -251,7 +259,7 @@ int eddlb200_resize(int dev, const float *a, float *b, int n, int c, int ah, int
     if (!total) return 0;
     EB_READS(a, (size_t)n * c * ah * aw * sizeof(float)); EB_WRITES(b, total * sizeof(float));
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * total);
-    scale_kernel<<<grid_for(total, kBlock), kBlock, 0, st>>>(a, b, total, g);
+    eb::launch(scale_kernel, grid_for(total, kBlock), kBlock, 0, st, a, b, total, g);
     EB_LAUNCH_CHECK("gpu_scale");
     return 0;
 }
@@ -265,7 +273,7 @@ int eddlb200_resize_bwd(int dev, float *a_delta, const float *b_delta, int n, in
     if (!total) return 0;
     EB_READS(b_delta, (size_t)n * c * bh * bw * sizeof(float)); EB_MODIFIES(a_delta, total * sizeof(float));
     ProfScope prof(cx, PROF_ELEMENTWISE, 8.0 * total + 4.0 * n * c * bh * bw);
-    scale_bwd_kernel<<<grid_for(total, kBlock), kBlock, 0, st>>>(a_delta, b_delta, total, g);
+    eb::launch(scale_bwd_kernel, grid_for(total, kBlock), kBlock, 0, st, a_delta, b_delta, total, g);
     EB_LAUNCH_CHECK("gpu_scale_back");
     return 0;
 }
@@ -276,7 +284,7 @@ int eddlb200_rand_binary(int dev, float *a, size_t n, float p, size_t seed, size
     EB_REQUIRE(a, "gpu_rand_binary");
     EB_WRITES(a, n * sizeof(float));
     ProfScope prof(cx, PROF_ELEMENTWISE, 4.0 * n);
-    rand_binary_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(a, n, p, (unsigned long long)seed, (unsigned long long)offset);
+    eb::launch(rand_binary_kernel, grid_for(n, kBlock), kBlock, 0, st, a, n, p, (unsigned long long)seed, (unsigned long long)offset);
     EB_LAUNCH_CHECK("gpu_rand_binary");
     return 0;
 }

@@ -20,6 +20,7 @@ constexpr int BM = 64, BN = 64, BK = 16, TB = 256;
 __global__ void __launch_bounds__(TB) sgemm_kernel(const float *__restrict__ A, int ta, const float *__restrict__ B, int tb,
                                                    float *__restrict__ C, int inc_c, int m, int n, int k, int k_per_split,
                                                    float *__restrict__ part) {
+    EB_GRID_WAIT();
     __shared__ float As[BK][BM + 4];
     __shared__ float Bs[BK][BN + 4];
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(TB) sgemm_kernel(const float *__restrict__ A, 
 
 // c[i] = (inc_c ? c[i] : 0) + part[0][i] + part[1][i] + ...   (fixed order)
 __global__ void __launch_bounds__(256) sgemm_combine_kernel(const float *__restrict__ part, float *__restrict__ c, size_t count, int splits, int inc_c) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
         float v = inc_c ? c[i] : 0.f;
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(256) sgemm_combine_kernel(const float *__restr
 }
 
 __global__ void __launch_bounds__(256) rowbias_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ c, size_t total, int cols) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += stride) c[p] = __fadd_rn(a[p], __ldg(b + (p % cols)));
 }
@@ -93,6 +96,7 @@ __global__ void __launch_bounds__(256) rowbias_kernel(const float *__restrict__ 
 // axis 0: one thread per column walks the rows in order (the reference's order), coalesced
 // across columns.  axis 1: one warp per row.
 __global__ void __launch_bounds__(256) colsum_kernel(const float *__restrict__ a, float *__restrict__ b, int rows, int cols, int inc_b) {
+    EB_GRID_WAIT();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cols) return;
     float s = inc_b ? b[j] : 0.f;
@@ -100,6 +104,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float *__restrict__ a
     b[j] = s;
 }
 __global__ void __launch_bounds__(256) rowsum_kernel(const float *__restrict__ a, float *__restrict__ b, int rows, int cols, int inc_b) {
+    EB_GRID_WAIT();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -143,7 +148,7 @@ int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, flo
         if (splits < 1) splits = 1;
     }
     if (splits == 1) {
-        sgemm_kernel<<<grid, TB, 0, st>>>(a, ta, b, tb, c, inc_c, m, n, k, k, nullptr);
+        eb::launch(sgemm_kernel, grid, TB, 0, st, a, ta, b, tb, c, inc_c, m, n, k, k, nullptr);
         EB_LAUNCH_CHECK("gpu_mult2D");
         return 0;
     }
@@ -154,9 +159,9 @@ int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, flo
     float *part = (float *)scratch(cx, count * splits * sizeof(float));
     if (!part) return cudaErrorMemoryAllocation;
     grid.z = splits;
-    sgemm_kernel<<<grid, TB, 0, st>>>(a, ta, b, tb, c, inc_c, m, n, k, kps, part);
+    eb::launch(sgemm_kernel, grid, TB, 0, st, a, ta, b, tb, c, inc_c, m, n, k, kps, part);
     EB_LAUNCH_CHECK("gpu_mult2D");
-    sgemm_combine_kernel<<<grid_for(count, 256), 256, 0, st>>>(part, c, count, splits, inc_c == 1);
+    eb::launch(sgemm_combine_kernel, grid_for(count, 256), 256, 0, st, part, c, count, splits, inc_c == 1);
     EB_LAUNCH_CHECK("gpu_mult2D(combine)");
     return 0;
 }
@@ -168,7 +173,7 @@ int eddlb200_sum2d_rowwise(int dev, const float *a, const float *b, float *c, in
     if (!total) return 0;
     EB_READS(a, total * sizeof(float)); EB_READS(b, (size_t)cols * sizeof(float));
     if (c != a) EB_WRITES(c, total * sizeof(float));
-    rowbias_kernel<<<grid_for(total, 256), 256, 0, st>>>(a, b, c, total, cols);
+    eb::launch(rowbias_kernel, grid_for(total, 256), 256, 0, st, a, b, c, total, cols);
     EB_LAUNCH_CHECK("gpu_sum2D_rowwise");
     return 0;
 }
@@ -180,10 +185,10 @@ int eddlb200_reduce_sum2d(int dev, const float *a, float *b, int rows, int cols,
     if (inc_b) EB_MODIFIES(b, (size_t)(axis == 0 ? cols : rows) * sizeof(float)); else EB_WRITES(b, (size_t)(axis == 0 ? cols : rows) * sizeof(float));
     if (axis == 0) {
         if (!cols) return 0;
-        colsum_kernel<<<(cols + 255) / 256, 256, 0, st>>>(a, b, rows, cols, inc_b);
+        eb::launch(colsum_kernel, (cols + 255) / 256, 256, 0, st, a, b, rows, cols, inc_b);
     } else {
         if (!rows) return 0;
-        rowsum_kernel<<<(rows + 7) / 8, 256, 0, st>>>(a, b, rows, cols, inc_b);
+        eb::launch(rowsum_kernel, (rows + 7) / 8, 256, 0, st, a, b, rows, cols, inc_b);
     }
     EB_LAUNCH_CHECK("gpu_reduce_sum2D");
     return 0;

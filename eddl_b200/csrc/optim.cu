@@ -23,6 +23,7 @@ __device__ __forceinline__ void sgd_one(float &p, float g, float &m, float lr, f
 }
 
 __global__ void __launch_bounds__(kBlock) sgd_kernel(float *p, const float *g, float *m, float lr, float mu, size_t n4, size_t n) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     for (size_t j = i; j < n4; j += stride) {
@@ -44,6 +45,7 @@ struct Chunk { unsigned tensor; unsigned offset_k; };   // offset in units of kC
 constexpr unsigned kChunk = 16384;
 
 __global__ void __launch_bounds__(kBlock) sgd_multi_kernel(const TensorRef *__restrict__ tensors, const Chunk *__restrict__ chunks, int nchunks, float lr, float mu) {
+    EB_GRID_WAIT();
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const Chunk ch = chunks[c];
         const TensorRef t = tensors[ch.tensor];
@@ -87,6 +89,7 @@ struct AdamRef { float *p, *g, *m, *v; unsigned long long n; };
 // Multi-tensor Adam: the same chunk table as sgd_multi_kernel, 28 bytes per parameter plus the squared gradient the
 // reference leaves in the gradient tensor.
 __global__ void __launch_bounds__(kBlock) adam_multi_kernel(const AdamRef *__restrict__ tensors, const Chunk *__restrict__ chunks, int nchunks, AdamCoef k) {
+    EB_GRID_WAIT();
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const Chunk ch = chunks[c];
         const AdamRef t = tensors[ch.tensor];
@@ -126,6 +129,7 @@ AdamCoef adam_coef(float lr, float beta1, float beta2, float eps, int t) {
 
 __global__ void __launch_bounds__(kBlock) adam_kernel(float *p, float *g, float *m, float *v, float lr, float b1, float b2, float omb1, float omb2,
                                                       float bc1, float bc2, float eps, size_t n) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
         const float gj = g[j];
@@ -159,7 +163,7 @@ int eddlb200_sgd_momentum(int dev, float *p, const float *g, float *m, float lr,
     EB_MODIFIES(p, n * sizeof(float)); EB_READS(g, n * sizeof(float)); EB_MODIFIES(m, n * sizeof(float));
     const bool vec = aligned16(p) && aligned16(g) && aligned16(m);
     const size_t n4 = vec ? n / 4 : 0;
-    sgd_kernel<<<grid_for(vec ? (n4 ? n4 : 1) : n, kBlock), kBlock, 0, st>>>(p, g, m, lr, mu, n4, n);
+    eb::launch(sgd_kernel, grid_for(vec ? (n4 ? n4 : 1) : n, kBlock), kBlock, 0, st, p, g, m, lr, mu, n4, n);
     EB_LAUNCH_CHECK("sgd_momentum");
     return 0;
 }
@@ -195,7 +199,7 @@ int eddlb200_sgd_momentum_multi(int dev, float *const *p, const float *const *g,
     // pageable source: cudaMemcpyAsync returns after staging, so `host` may go out of scope
     int blocks = (int)chunks.size();
     if (blocks > EDDLB200_NUM_SMS * 8) blocks = EDDLB200_NUM_SMS * 8;
-    sgd_multi_kernel<<<blocks, kBlock, 0, st>>>((const TensorRef *)tab, (const Chunk *)(tab + off_c), (int)chunks.size(), lr, mu);
+    eb::launch(sgd_multi_kernel, blocks, kBlock, 0, st, (const TensorRef *)tab, (const Chunk *)(tab + off_c), (int)chunks.size(), lr, mu);
     EB_LAUNCH_CHECK("sgd_momentum_multi");
     return 0;
 }
@@ -206,7 +210,7 @@ int eddlb200_adam(int dev, float *p, float *g, float *m, float *v, float lr, flo
     EB_REQUIRE(p && g && m && v && t >= 1, "adam");
     EB_MODIFIES(p, n * sizeof(float)); EB_MODIFIES(g, n * sizeof(float)); EB_MODIFIES(m, n * sizeof(float)); EB_MODIFIES(v, n * sizeof(float));
     const AdamCoef k = adam_coef(lr, beta1, beta2, eps, t);
-    adam_kernel<<<grid_for(n, kBlock), kBlock, 0, st>>>(p, g, m, v, lr, beta1, beta2, k.omb1, k.omb2, k.bc1, k.bc2, eps, n);
+    eb::launch(adam_kernel, grid_for(n, kBlock), kBlock, 0, st, p, g, m, v, lr, beta1, beta2, k.omb1, k.omb2, k.bc1, k.bc2, eps, n);
     EB_LAUNCH_CHECK("adam");
     return 0;
 }
@@ -241,7 +245,7 @@ int eddlb200_adam_multi(int dev, float *const *p, float *const *g, float *const 
     if (e != cudaSuccess) return cuda_status(e, "adam_multi(table)");
     int blocks = (int)chunks.size();
     if (blocks > EDDLB200_NUM_SMS * 8) blocks = EDDLB200_NUM_SMS * 8;
-    adam_multi_kernel<<<blocks, kBlock, 0, st>>>((const AdamRef *)tab, (const Chunk *)(tab + off_c), (int)chunks.size(), adam_coef(lr, beta1, beta2, eps, t));
+    eb::launch(adam_multi_kernel, blocks, kBlock, 0, st, (const AdamRef *)tab, (const Chunk *)(tab + off_c), (int)chunks.size(), adam_coef(lr, beta1, beta2, eps, t));
     EB_LAUNCH_CHECK("adam_multi");
     return 0;
 }

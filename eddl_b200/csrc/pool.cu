@@ -29,6 +29,7 @@ template <int KR, int KC, typename IDX>
 __global__ void __launch_bounds__(kBlock) maxpool_fwd_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                              float *__restrict__ ind_x, float *__restrict__ ind_y,
                                                              size_t total, PoolGeom g) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const int kr = KR > 0 ? KR : g.kr, kc = KC > 0 ? KC : g.kc;
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += stride) {
@@ -74,6 +75,7 @@ __global__ void __launch_bounds__(kBlock) maxpool_fwd_kernel(const float *__rest
 
 template <typename IDX>
 __global__ void __launch_bounds__(kBlock) avgpool_fwd_kernel(const float *__restrict__ in, float *__restrict__ out, size_t total, PoolGeom g) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const float ksize = (float)(g.kr * g.kc);
     for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += stride) {
@@ -116,6 +118,7 @@ template <bool MAX, typename IDX>
 __global__ void __launch_bounds__(kBlock) pool_bwd_kernel(const float *__restrict__ d, const float *__restrict__ ind_x,
                                                           const float *__restrict__ ind_y, float *__restrict__ id,
                                                           size_t total_in, PoolGeom g, int id_zero) {
+    EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const float ksize = (float)(g.kr * g.kc);
     for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total_in; q += stride) {
@@ -182,6 +185,7 @@ __global__ void __launch_bounds__(kBlock) pool_bwd_kernel(const float *__restric
 __global__ void __launch_bounds__(256) maxpool_bwd_plane_kernel(const float *__restrict__ d, const float *__restrict__ ind_x,
                                                                 const float *__restrict__ ind_y, float *__restrict__ id,
                                                                 unsigned planes, PoolGeom g, int id_zero) {
+    EB_GRID_WAIT();
     extern __shared__ float sm_pool[];
     const int opl = g.oh * g.ow, ipl = g.ih * g.iw;
     float *sd = sm_pool;
@@ -308,10 +312,10 @@ int eddlb200_maxpool2d_fwd(int dev, const float *in, float *out, float *ind_x, f
     EB_WRITES(out, total * sizeof(float)); EB_WRITES(ind_x, total * sizeof(float)); EB_WRITES(ind_y, total * sizeof(float));
     ProfScope prof(cx, PROF_POOL, 4.0 * n * c * ih * iw + 12.0 * total);
     const int blocks = grid_for(total, kBlock);
-    if ((size_t)n * c * ih * iw >= (size_t(1) << 32)) maxpool_fwd_kernel<0, 0, size_t><<<blocks, kBlock, 0, st>>>(in, out, ind_x, ind_y, total, g);
-    else if (kr == 2 && kc == 2) maxpool_fwd_kernel<2, 2, unsigned><<<blocks, kBlock, 0, st>>>(in, out, ind_x, ind_y, total, g);
-    else if (kr == 3 && kc == 3) maxpool_fwd_kernel<3, 3, unsigned><<<blocks, kBlock, 0, st>>>(in, out, ind_x, ind_y, total, g);
-    else maxpool_fwd_kernel<0, 0, unsigned><<<blocks, kBlock, 0, st>>>(in, out, ind_x, ind_y, total, g);
+    if ((size_t)n * c * ih * iw >= (size_t(1) << 32)) eb::launch(maxpool_fwd_kernel<0, 0, size_t>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
+    else if (kr == 2 && kc == 2) eb::launch(maxpool_fwd_kernel<2, 2, unsigned>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
+    else if (kr == 3 && kc == 3) eb::launch(maxpool_fwd_kernel<3, 3, unsigned>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
+    else eb::launch(maxpool_fwd_kernel<0, 0, unsigned>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
     EB_LAUNCH_CHECK("gpu_mpool2D");
     return 0;
 }
@@ -343,12 +347,12 @@ int eddlb200_maxpool2d_bwd(int dev, const float *d, const float *ind_x, const fl
         if (per_sm > 8) per_sm = 8;
         if (per_sm < 1) per_sm = 1;
         unsigned blocks = planes < (unsigned)(EDDLB200_NUM_SMS * per_sm) ? planes : (unsigned)(EDDLB200_NUM_SMS * per_sm);
-        maxpool_bwd_plane_kernel<<<blocks, 256, plane_smem, st>>>(d, ind_x, ind_y, id, planes, g, id_zero);
+        eb::launch(maxpool_bwd_plane_kernel, blocks, 256, plane_smem, st, d, ind_x, ind_y, id, planes, g, id_zero);
         EB_LAUNCH_CHECK("gpu_mpool2D_back");
         return 0;
     }
-    if (total < (size_t(1) << 32)) pool_bwd_kernel<true, unsigned><<<grid_for(total, kBlock), kBlock, 0, st>>>(d, ind_x, ind_y, id, total, g, id_zero);
-    else pool_bwd_kernel<true, size_t><<<grid_for(total, kBlock), kBlock, 0, st>>>(d, ind_x, ind_y, id, total, g, id_zero);
+    if (total < (size_t(1) << 32)) eb::launch(pool_bwd_kernel<true, unsigned>, grid_for(total, kBlock), kBlock, 0, st, d, ind_x, ind_y, id, total, g, id_zero);
+    else eb::launch(pool_bwd_kernel<true, size_t>, grid_for(total, kBlock), kBlock, 0, st, d, ind_x, ind_y, id, total, g, id_zero);
     EB_LAUNCH_CHECK("gpu_mpool2D_back");
     return 0;
 }
@@ -364,8 +368,8 @@ int eddlb200_avgpool2d_fwd(int dev, const float *in, float *out, int n, int c, i
     EB_READS(in, (size_t)n * c * ih * iw * sizeof(float));
     EB_WRITES(out, total * sizeof(float));
     ProfScope prof(cx, PROF_POOL, 4.0 * n * c * ih * iw + 4.0 * total);
-    if ((size_t)n * c * ih * iw < (size_t(1) << 32)) avgpool_fwd_kernel<unsigned><<<grid_for(total, kBlock), kBlock, 0, st>>>(in, out, total, g);
-    else avgpool_fwd_kernel<size_t><<<grid_for(total, kBlock), kBlock, 0, st>>>(in, out, total, g);
+    if ((size_t)n * c * ih * iw < (size_t(1) << 32)) eb::launch(avgpool_fwd_kernel<unsigned>, grid_for(total, kBlock), kBlock, 0, st, in, out, total, g);
+    else eb::launch(avgpool_fwd_kernel<size_t>, grid_for(total, kBlock), kBlock, 0, st, in, out, total, g);
     EB_LAUNCH_CHECK("gpu_avgpool2D");
     return 0;
 }
@@ -383,8 +387,8 @@ int eddlb200_avgpool2d_bwd(int dev, const float *d, float *id, int n, int c, int
     EB_NOTES(id, total * sizeof(float));
     if (lz_any(cx) && id != d) { int status = 0; id_zero = lz_take(cx, st, id, total * sizeof(float), &status); if (status) return status; }
     ProfScope prof(cx, PROF_POOL, 4.0 * n * c * oh * ow + (id_zero ? 4.0 : 8.0) * total);
-    if (total < (size_t(1) << 32)) pool_bwd_kernel<false, unsigned><<<grid_for(total, kBlock), kBlock, 0, st>>>(d, nullptr, nullptr, id, total, g, id_zero);
-    else pool_bwd_kernel<false, size_t><<<grid_for(total, kBlock), kBlock, 0, st>>>(d, nullptr, nullptr, id, total, g, id_zero);
+    if (total < (size_t(1) << 32)) eb::launch(pool_bwd_kernel<false, unsigned>, grid_for(total, kBlock), kBlock, 0, st, d, nullptr, nullptr, id, total, g, id_zero);
+    else eb::launch(pool_bwd_kernel<false, size_t>, grid_for(total, kBlock), kBlock, 0, st, d, nullptr, nullptr, id, total, g, id_zero);
     EB_LAUNCH_CHECK("gpu_avgpool2D_back");
     return 0;
 }

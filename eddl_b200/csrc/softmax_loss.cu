@@ -20,6 +20,7 @@ constexpr int kWarpsPerBlock = kBlock / 32;
 
 // sample si of an [outer, cols, inner] view starts at (si / inner)*cols*inner + si % inner
 __global__ void __launch_bounds__(kBlock) softmax_fwd_kernel(const float *__restrict__ a, float *__restrict__ b, int nsamples, int cols, int inner) {
+    EB_GRID_WAIT();
     const int lane = threadIdx.x & 31;
     for (int si = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); si < nsamples; si += gridDim.x * kWarpsPerBlock) {
         const size_t base = (size_t)(si / inner) * cols * inner + (si % inner);
@@ -46,6 +47,7 @@ __global__ void __launch_bounds__(kBlock) softmax_fwd_kernel(const float *__rest
 // dot = sum_j d[j]*s[j]:  pd[i] += d[i]*s[i] - s[i]*dot  (same value up to summation order).
 __global__ void __launch_bounds__(kBlock) softmax_bwd_kernel(const float *__restrict__ d, const float *__restrict__ s, float *__restrict__ pd,
                                                              int nsamples, int cols, int inner) {
+    EB_GRID_WAIT();
     const int lane = threadIdx.x & 31;
     for (int si = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); si < nsamples; si += gridDim.x * kWarpsPerBlock) {
         const size_t base = (size_t)(si / inner) * cols * inner + (si % inner);
@@ -62,6 +64,7 @@ __global__ void __launch_bounds__(kBlock) softmax_bwd_kernel(const float *__rest
 
 // out[0] += sum over this block's rows of sum_c y*logf(p + 1e-7)
 __global__ void __launch_bounds__(kBlock) cce_value_kernel(const float *__restrict__ y, const float *__restrict__ p, int rows, int cols, float *out) {
+    EB_GRID_WAIT();
     __shared__ float sm[32];
     const int lane = threadIdx.x & 31;
     float acc = 0.f;
@@ -79,6 +82,7 @@ __global__ void __launch_bounds__(kBlock) cce_value_kernel(const float *__restri
 }
 
 __global__ void __launch_bounds__(kBlock) accuracy_kernel(const float *__restrict__ y, const float *__restrict__ p, int rows, int cols, int *out) {
+    EB_GRID_WAIT();
     const int lane = threadIdx.x & 31;
     int hits = 0;
     for (int r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); r < rows; r += gridDim.x * kWarpsPerBlock) {
@@ -122,7 +126,7 @@ int eddlb200_softmax_fwd_nd(int dev, const float *a, float *b, int outer, int co
     if (!ns) return 0;
     EB_READS(a, (size_t)ns * cols * sizeof(float));
     if (b != a) EB_WRITES(b, (size_t)ns * cols * sizeof(float));
-    softmax_fwd_kernel<<<grid_for((size_t)ns * 32, kBlock), kBlock, 0, st>>>(a, b, (int)ns, cols, inner);
+    eb::launch(softmax_fwd_kernel, grid_for((size_t)ns * 32, kBlock), kBlock, 0, st, a, b, (int)ns, cols, inner);
     EB_LAUNCH_CHECK("gpu_full_softmax");
     return 0;
 }
@@ -134,7 +138,7 @@ int eddlb200_softmax_bwd_nd(int dev, const float *d, const float *s, float *pd, 
     EB_REQUIRE(ns < 0x7fffffffLL, "gpu_d_full_softmax");
     if (!ns) return 0;
     EB_READS(d, (size_t)ns * cols * sizeof(float)); EB_READS(s, (size_t)ns * cols * sizeof(float)); EB_MODIFIES(pd, (size_t)ns * cols * sizeof(float));
-    softmax_bwd_kernel<<<grid_for((size_t)ns * 32, kBlock), kBlock, 0, st>>>(d, s, pd, (int)ns, cols, inner);
+    eb::launch(softmax_bwd_kernel, grid_for((size_t)ns * 32, kBlock), kBlock, 0, st, d, s, pd, (int)ns, cols, inner);
     EB_LAUNCH_CHECK("gpu_d_full_softmax");
     return 0;
 }
@@ -154,9 +158,9 @@ static int loss_and_hits(DevCtx *cx, cudaStream_t st, const float *y_true, const
     cudaError_t e = cudaMemsetAsync(dsc, 0, 2 * sizeof(float), st);
     if (e != cudaSuccess) return cuda_status(e, "gpu_categorical_cross_entropy");
     if (rows) {
-        cce_value_kernel<<<((size_t)rows * cols <= (size_t(1) << 20)) ? 1 : grid_for((size_t)rows * 32, kBlock, 1), kBlock, 0, st>>>(y_true, y_pred, rows, cols, dsc);
+        eb::launch(cce_value_kernel, ((size_t)rows * cols <= (size_t(1) << 20)) ? 1 : grid_for((size_t)rows * 32, kBlock, 1), kBlock, 0, st, y_true, y_pred, rows, cols, dsc);
         EB_LAUNCH_CHECK("gpu_categorical_cross_entropy");
-        accuracy_kernel<<<grid_for((size_t)rows * 32, kBlock, 1), kBlock, 0, st>>>(y_true, y_pred, rows, cols, (int *)(dsc + 1));
+        eb::launch(accuracy_kernel, grid_for((size_t)rows * 32, kBlock, 1), kBlock, 0, st, y_true, y_pred, rows, cols, (int *)(dsc + 1));
         EB_LAUNCH_CHECK("gpu_accuracy");
     }
     e = cudaMemcpyAsync(hsc, dsc, 2 * sizeof(float), cudaMemcpyDeviceToHost, st);
