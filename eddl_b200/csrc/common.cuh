@@ -28,7 +28,15 @@ cudaEvent_t handoff_event(DevCtx *c);
 void *scratch(DevCtx *c, size_t bytes);
 // Pinned host words + device words used to return scalars (loss, accuracy).
 float *host_scalars(DevCtx *c);    // 64 floats
-float *dev_scalars(DevCtx *c);     // 64 floats
+float *dev_scalars(DevCtx *c);     // kDevScalars floats
+constexpr int kDevScalars = 1024;
+// `count` device words that are zero whenever no kernel is using them: a kernel whose blocks count their arrivals in them (the last
+// one combines what the others left) puts the zeros back.  Shared by all kernels of the device's compute stream.
+unsigned *tickets(DevCtx *c, size_t count);
+// Device copy of a small host table (the tensor lists of the multi-tensor calls).  A training loop passes the same lists step
+// after step, so the last sixteen tables are kept and an unchanged one is not uploaded again.  Valid on the compute stream
+// until sixteen other tables have been asked for.
+const char *device_table(DevCtx *c, cudaStream_t st, const char *host, size_t bytes);
 ncclComm *comm_of(DevCtx *c);
 int comm_nranks(DevCtx *c);
 void count_launch(DevCtx *c, unsigned n = 1);

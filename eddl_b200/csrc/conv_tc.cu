@@ -1479,18 +1479,24 @@ const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::arr
     }
     const size_t packed_bytes = (size_t)kblocks * tiles_n * bn * BK * sizeof(float) * (precision != 1 ? 2 : 1);
     if (slot < 0) {
-        // a new image: take a free slot, or the slot of an image whose tensor is gone (released memory is no longer observed)
-        if ((int)pc.entries.size() < kMaxPackJobs) { pc.entries.push_back(PackEntry{}); slot = (int)pc.entries.size() - 1; }
-        else {
-            for (size_t i = 0; i < pc.entries.size() && slot < 0; i++)
-                if (watch_version(cx, pc.entries[i].src) == 0) slot = (int)i;
+        // A new image.  The memory of an image of the same size whose tensor is gone (released memory is no longer observed) is taken
+        // over as it is: kernels that still read it come first on the stream.  Otherwise a free slot, or the slot of any image that is gone.
+        int gone = -1;
+        for (size_t i = 0; i < pc.entries.size() && slot < 0; i++) {
+            if (watch_version(cx, pc.entries[i].src) != 0) continue;
+            if (pc.entries[i].packed && pc.entries[i].packed_bytes == packed_bytes) slot = (int)i;
+            else if (gone < 0) gone = (int)i;
+        }
+        if (slot < 0 && (int)pc.entries.size() < kMaxPackJobs) { pc.entries.push_back(PackEntry{}); slot = (int)pc.entries.size() - 1; }
+        if (slot < 0) {
+            slot = gone;
             if (slot < 0) return nullptr;
             cudaStreamSynchronize(st);                  // kernels already enqueued may still read the old image
             cudaFree(pc.entries[slot].packed);
             pc.entries[slot] = PackEntry{};
         }
         PackEntry &e = pc.entries[slot];
-        if (cudaMalloc((void **)&e.packed, packed_bytes) != cudaSuccess) { cudaGetLastError(); e = PackEntry{}; return nullptr; }
+        if (!e.packed && cudaMalloc((void **)&e.packed, packed_bytes) != cudaSuccess) { cudaGetLastError(); e = PackEntry{}; return nullptr; }
         e.tkey = tkey; e.bn = bn; e.precision = precision; e.src = src; e.src_bytes = src_bytes; e.packed_bytes = packed_bytes;
         e.blocks = (unsigned)kblocks * (unsigned)tiles_n; e.version = 0;
         const PackJob job{src, rowB, kB, e.packed, bn, n_total, tiles_n, row_fastest, precision, kblocks};

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kBlock) pad_kernel(float *a, float *b, unsigne
     }
 }
 
-// Many fills in one launch: segment table in the scratch arena, one block-chunk of 16K elements per table entry.
+// Many fills in one launch: one block-chunk of 16K elements per table entry.
 struct FillSeg { float *p; unsigned long long n; float v; unsigned pad; };
 struct FillChunk { unsigned seg; unsigned offset_k; };
 constexpr unsigned kFillChunk = 16384;
@@ -286,13 +286,11 @@ int eddlb200_fill_multi(int dev, float *const *ptrs, const size_t *sizes, const 
     }
     if (chunks.empty()) return 0;
     const size_t bytes_s = segs.size() * sizeof(FillSeg), off_c = (bytes_s + 255) & ~size_t(255), bytes_c = chunks.size() * sizeof(FillChunk);
-    char *tab = (char *)scratch(cx, off_c + bytes_c);
-    if (!tab) return cudaErrorMemoryAllocation;
     std::vector<char> host(off_c + bytes_c);
     memcpy(host.data(), segs.data(), bytes_s);
     memcpy(host.data() + off_c, chunks.data(), bytes_c);
-    cudaError_t e = cudaMemcpyAsync(tab, host.data(), host.size(), cudaMemcpyHostToDevice, st);   // pageable source: staged before return
-    if (e != cudaSuccess) return cuda_status(e, "fill_multi(table)");
+    const char *tab = device_table(cx, st, host.data(), host.size());
+    if (!tab) return cudaErrorMemoryAllocation;
     ProfScope prof(cx, PROF_ELEMENTWISE, 4.0 * total);
     int blocks = (int)chunks.size();
     if (blocks > EDDLB200_NUM_SMS * 8) blocks = EDDLB200_NUM_SMS * 8;

@@ -3,10 +3,9 @@
 // gpu_sum2D_rowwise (gpu_math.cu:517-528) and gpu_reduce_sum2D (gpu_reduction.cu:232-244,
 // one atomicAdd per element); arithmetic as cpu_mult2D / cpu_sum2D_rowwise /
 // cpu_reduce_sum2D (src/hardware/cpu/cpu_math.cpp:302-325,369-380; cpu_reduction.cpp:91-112).
-// The dense layers of the convnets are small (<= 64x2048x1000), so this is an fp32
-// FMA kernel: 64x64 block tile, 16-deep k slices staged in shared memory, 4x4
-// accumulators per thread, exact fp32 accumulation.  When the output has fewer tiles than the GPU has SMs (batch 64:
-// 16 or 32 tiles) the k range is split across blockIdx.z and the partials are combined in a fixed order.
+// The dense layers of the nets are small (64 x 2048 x 1000), so this is an fp32 FMA
+// kernel; see sgemm_kernel.
+#include <cooperative_groups.h>
 #include "common.cuh"
 #include "conv_common.cuh"
 
@@ -14,83 +13,124 @@ namespace {
 
 using namespace eb;
 
-constexpr int BM = 64, BN = 64, BK = 16, TB = 256;
+constexpr int BM = 64, BN = 64, BK = 32, TB = 256;
+constexpr int kMaxCluster = 8;          // portable cluster size: k slices of one output tile
 
-// Row-major storage.  A: ta ? [k,m] : [m,k]; B: tb ? [n,k] : [k,n]; C: [m,n].
-__global__ void __launch_bounds__(TB) sgemm_kernel(const float *__restrict__ A, int ta, const float *__restrict__ B, int tb,
-                                                   float *__restrict__ C, int inc_c, int m, int n, int k, int k_per_split,
-                                                   float *__restrict__ part) {
+// Row-major storage.  A: TA ? [k,m] : [m,k]; B: TB_ ? [n,k] : [k,n]; C: [m,n].
+// The products of the nets are small (100 x 1024 x 1024): what bounds them is not arithmetic but how much of the GPU takes part
+// and how long the chain load -> multiply -> combine is.  A 64 x 64 tile is computed by a CLUSTER of up to eight blocks, each
+// with its own slice of k; the partial tiles meet in the blocks' shared memory, and every block adds its share of the rows from
+// all of them in slice order and stores it -- one launch, no partial sums in memory.  A k step of 32 is fetched into registers
+// while the one before it is multiplied (16-byte loads where VEC: rows and pointers 16-byte aligned), 4 x 4 outputs per
+// thread.  100 x 1024 x 1024: 30 us (tensor-core kernel with split-K and operand packing) -> 8 us; exact fp32.
+template <bool TA, bool TB_, bool VEC>
+__global__ void __launch_bounds__(TB) sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, int inc_c,
+                                                   int m, int n, int k, int k_per_slice) {
+    constexpr int LD = BM + 4;
+    __shared__ __align__(16) float smem[2 * BK * LD];                 // As and Bs; afterwards the 64 x 64 partial tile
+    float (*As)[LD] = reinterpret_cast<float (*)[LD]>(smem), (*Bs)[LD] = reinterpret_cast<float (*)[LD]>(smem + BK * LD);
     EB_GRID_WAIT();
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int kbeg = blockIdx.z * k_per_slice, kend = min(k, kbeg + k_per_slice);
     float acc[4][4] = {};
-    const int kbeg = blockIdx.z * k_per_split;
-    int kend = k;
-    if (part) { kend = min(k, kbeg + k_per_split); C = part + (size_t)blockIdx.z * m * n; inc_c = 0; }
+    // An operand tile is 64 x BK = 512 pieces of four elements along the dimension that is contiguous in memory; a thread moves
+    // pieces threadIdx.x and threadIdx.x + 256.  K_FAST: contiguous along k (8 pieces per row), else along the row (16 per k).
+    auto fetch = [&](const float *src, bool k_fast, int rows, int row0, int ld, int k0, int piece) -> float4 {
+        const int r = k_fast ? piece / (BK / 4) : (piece % 16) * 4, kk = k_fast ? (piece % (BK / 4)) * 4 : piece / 16;
+        const int gr = row0 + r, gk = k0 + kk;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k_fast) {
+            if (gr < rows) {
+                const float *q = src + (size_t)gr * ld + gk;
+                if (VEC && gk + 4 <= kend) v = ldg4(q);
+                else { if (gk < kend) v.x = __ldg(q); if (gk + 1 < kend) v.y = __ldg(q + 1); if (gk + 2 < kend) v.z = __ldg(q + 2); if (gk + 3 < kend) v.w = __ldg(q + 3); }
+            }
+        } else if (gk < kend) {
+            const float *q = src + (size_t)gk * ld + gr;
+            if (VEC && gr + 4 <= rows) v = ldg4(q);
+            else { if (gr < rows) v.x = __ldg(q); if (gr + 1 < rows) v.y = __ldg(q + 1); if (gr + 2 < rows) v.z = __ldg(q + 2); if (gr + 3 < rows) v.w = __ldg(q + 3); }
+        }
+        return v;
+    };
+    auto put = [&](float (*tile)[LD], bool k_fast, int piece, float4 v) {
+        if (k_fast) {
+            const int r = piece / (BK / 4), kk = (piece % (BK / 4)) * 4;
+            tile[kk][r] = v.x; tile[kk + 1][r] = v.y; tile[kk + 2][r] = v.z; tile[kk + 3][r] = v.w;
+        } else *reinterpret_cast<float4 *>(&tile[piece / 16][(piece % 16) * 4]) = v;
+    };
+    float4 a0, a1, b0, b1;
+    auto load = [&](int k0) {
+        a0 = fetch(A, !TA, m, m0, TA ? m : k, k0, threadIdx.x); a1 = fetch(A, !TA, m, m0, TA ? m : k, k0, threadIdx.x + TB);
+        b0 = fetch(B, TB_, n, n0, TB_ ? k : n, k0, threadIdx.x); b1 = fetch(B, TB_, n, n0, TB_ ? k : n, k0, threadIdx.x + TB);
+    };
+    load(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        for (int e = threadIdx.x; e < BM * BK; e += TB) {
-            // choose the traversal that is contiguous in memory
-            int mi, ki;
-            if (ta) { mi = e % BM; ki = e / BM; } else { ki = e % BK; mi = e / BK; }
-            const int gm = m0 + mi, gk = k0 + ki;
-            float v = 0.f;
-            if (gm < m && gk < kend) v = ta ? A[(size_t)gk * m + gm] : A[(size_t)gm * k + gk];
-            As[ki][mi] = v;
-        }
-        for (int e = threadIdx.x; e < BN * BK; e += TB) {
-            int ni, ki;
-            if (tb) { ki = e % BK; ni = e / BK; } else { ni = e % BN; ki = e / BN; }
-            const int gn = n0 + ni, gk = k0 + ki;
-            float v = 0.f;
-            if (gn < n && gk < kend) v = tb ? B[(size_t)gn * k + gk] : B[(size_t)gk * n + gn];
-            Bs[ki][ni] = v;
-        }
+        put(As, !TA, threadIdx.x, a0); put(As, !TA, threadIdx.x + TB, a1);
+        put(Bs, TB_, threadIdx.x, b0); put(Bs, TB_, threadIdx.x + TB, b1);
         __syncthreads();
+        if (k0 + BK < kend) load(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+            const float4 a = *reinterpret_cast<const float4 *>(&As[kk][ty * 4]), b = *reinterpret_cast<const float4 *>(&Bs[kk][tx * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
         __syncthreads();
     }
+    auto store = [&](int gm, int gn, float v) {
+        float *c = C + (size_t)gm * n + gn;
+        *c = inc_c == 1 ? __fadd_rn(*c, v) : (inc_c == 2 ? __fadd_rn(0.f, v) : v);          // 2: c is known to hold zeros
+    };
+    const unsigned slices = gridDim.z;
+    if (slices == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= m) continue;
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= n) continue;
-            float *c = C + (size_t)gm * n + gn;
-            *c = inc_c == 1 ? __fadd_rn(*c, acc[i][j]) : (inc_c == 2 ? __fadd_rn(0.f, acc[i][j]) : acc[i][j]);     // 2: c is known to hold zeros
-        }
+            for (int j = 0; j < 4; j++)
+                if (m0 + ty * 4 + i < m && n0 + tx * 4 + j < n) store(m0 + ty * 4 + i, n0 + tx * 4 + j, acc[i][j]);
+        return;
     }
+    static_assert(BM * BN <= 2 * BK * LD, "the partial tile takes the place of the operand tiles");
+#pragma unroll
+    for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(smem + (ty * 4 + i) * BN + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    const float *peer[kMaxCluster];
+    for (unsigned z = 0; z < kMaxCluster; z++) peer[z] = cluster.map_shared_rank(smem, z < slices ? z : 0);
+    for (int e = (int)blockIdx.z * TB + threadIdx.x; e < BM * BN; e += (int)slices * TB) {
+        float v[kMaxCluster];
+#pragma unroll
+        for (unsigned z = 0; z < kMaxCluster; z++) v[z] = z < slices ? peer[z][e] : 0.f;
+        float s = v[0];
+#pragma unroll
+        for (unsigned z = 1; z < kMaxCluster; z++) if (z < slices) s = __fadd_rn(s, v[z]);
+        const int gm = m0 + e / BN, gn = n0 + e % BN;
+        if (gm < m && gn < n) store(gm, gn, s);
+    }
+    cluster.sync();                     // a block's shared memory outlives the reads of the others
 }
 
-// c[i] = (inc_c ? c[i] : 0) + part[0][i] + part[1][i] + ...   (fixed order)
-__global__ void __launch_bounds__(256) sgemm_combine_kernel(const float *__restrict__ part, float *__restrict__ c, size_t count, int splits, int inc_c) {
-    EB_GRID_WAIT();
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        float v = inc_c ? c[i] : 0.f;
-        for (int z = 0; z < splits; z++) v = __fadd_rn(v, part[(size_t)z * count + i]);
-        c[i] = v;
-    }
+template <bool TA, bool TB_, bool VEC>
+int launch_sgemm(DevCtx *cx, cudaStream_t st, const float *a, const float *b, float *c, int inc_c, int m, int n, int k, int slices, int kps) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = slices;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((n + BN - 1) / BN, (m + BM - 1) / BM, slices); cfg.blockDim = dim3(TB); cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, sgemm_kernel<TA, TB_, VEC>, a, b, c, inc_c, m, n, k, kps);
+    EB_LAUNCH_CHECK("gpu_mult2D");
+    return 0;
 }
 
 __global__ void __launch_bounds__(256) rowbias_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ c, size_t total, int cols) {
     EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += stride) c[p] = __fadd_rn(a[p], __ldg(b + (p % cols)));
+    for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total; p += stride)
+        c[p] = __fadd_rn(a[p], __ldg(b + (total < (size_t(1) << 32) ? (unsigned)p % (unsigned)cols : p % cols)));
 }
 
 // axis 0: one thread per column walks the rows in order (the reference's order), coalesced
@@ -100,7 +140,15 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float *__restrict__ a
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cols) return;
     float s = inc_b ? b[j] : 0.f;
-    for (int i = 0; i < rows; i++) s = __fadd_rn(s, a[(size_t)i * cols + j]);
+    int i = 0;
+    for (; i + 16 <= rows; i += 16) {               // sixteen loads in flight, added in order: one memory latency per sixteen rows
+        float v[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) v[r] = __ldg(a + (size_t)(i + r) * cols + j);
+#pragma unroll
+        for (int r = 0; r < 16; r++) s = __fadd_rn(s, v[r]);
+    }
+    for (; i < rows; i++) s = __fadd_rn(s, __ldg(a + (size_t)i * cols + j));
     b[j] = s;
 }
 __global__ void __launch_bounds__(256) rowsum_kernel(const float *__restrict__ a, float *__restrict__ b, int rows, int cols, int inc_b) {
@@ -132,38 +180,26 @@ int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, flo
     }
     if (inc_c == 1) EB_MODIFIES(c, (size_t)m * n * sizeof(float)); else EB_WRITES(c, (size_t)m * n * sizeof(float));
     ProfScope prof(cx, PROF_GEMM, 2.0 * m * (double)n * k);
-    // Large products (ResNet-50's 2048 x 1000 classifier at batch 64) run on the tensor-core kernel (3xTF32, like the
-    // convolutions).  Below 2^26 multiply-adds its extra launches (operand packing, split-K combine) cost more than they save
-    // (VGG-16-BN's 512 x 512 layers at batch 128 were 2 % of a step slower there), and a library forced to the FMA path stays here.
-    if (conv_tc_allowed() && k >= 32 && (double)m * n * k >= 67108864.0) {
+    // Products of 2^29 multiply-adds or more run on the tensor-core kernel (3xTF32, like the convolutions).  Below that its fixed cost
+    // -- packing an operand, index tables, the split-K combine -- is more than the FMA kernel takes for the whole product
+    // (64 x 1000 x 2048 for ResNet-50's classifier: 29 -> 11 us), and a library forced to the FMA path stays here.
+    if (conv_tc_allowed() && k >= 32 && (double)m * n * k >= 536870912.0) {
         const int r = conv_tc_gemm(cx, st, a, ta, b, tb, c, inc_c, m, n, k, 0);
         if (r != 1) return r;
     }
-    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
-    const int tiles = (int)(grid.x * grid.y);
-    int splits = 1;
-    if (tiles < EDDLB200_NUM_SMS) {
-        splits = (2 * EDDLB200_NUM_SMS + tiles - 1) / tiles;
-        if (splits > k / (4 * BK)) splits = k / (4 * BK);
-        if (splits < 1) splits = 1;
-    }
-    if (splits == 1) {
-        eb::launch(sgemm_kernel, grid, TB, 0, st, a, ta, b, tb, c, inc_c, m, n, k, k, nullptr);
-        EB_LAUNCH_CHECK("gpu_mult2D");
-        return 0;
-    }
-    int kps = (k + splits - 1) / splits;
+    // k slices: two blocks per SM where the tiles alone do not give them, slices of at least 64 (two k steps)
+    const long long tiles = (long long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
+    int slices = 1;
+    while (slices < kMaxCluster && tiles * slices * 2 <= 2 * EDDLB200_NUM_SMS && k >= slices * 2 * 64) slices *= 2;
+    int kps = (k + slices - 1) / slices;
     kps = (kps + BK - 1) / BK * BK;
-    splits = (k + kps - 1) / kps;
-    const size_t count = (size_t)m * n;
-    float *part = (float *)scratch(cx, count * splits * sizeof(float));
-    if (!part) return cudaErrorMemoryAllocation;
-    grid.z = splits;
-    eb::launch(sgemm_kernel, grid, TB, 0, st, a, ta, b, tb, c, inc_c, m, n, k, kps, part);
-    EB_LAUNCH_CHECK("gpu_mult2D");
-    eb::launch(sgemm_combine_kernel, grid_for(count, 256), 256, 0, st, part, c, count, splits, inc_c == 1);
-    EB_LAUNCH_CHECK("gpu_mult2D(combine)");
-    return 0;
+    const bool vec = aligned16(a) && aligned16(b) && (ta ? m : k) % 4 == 0 && (tb ? k : n) % 4 == 0;
+    if (ta) {
+        if (tb) return vec ? launch_sgemm<true, true, true>(cx, st, a, b, c, inc_c, m, n, k, slices, kps) : launch_sgemm<true, true, false>(cx, st, a, b, c, inc_c, m, n, k, slices, kps);
+        return vec ? launch_sgemm<true, false, true>(cx, st, a, b, c, inc_c, m, n, k, slices, kps) : launch_sgemm<true, false, false>(cx, st, a, b, c, inc_c, m, n, k, slices, kps);
+    }
+    if (tb) return vec ? launch_sgemm<false, true, true>(cx, st, a, b, c, inc_c, m, n, k, slices, kps) : launch_sgemm<false, true, false>(cx, st, a, b, c, inc_c, m, n, k, slices, kps);
+    return vec ? launch_sgemm<false, false, true>(cx, st, a, b, c, inc_c, m, n, k, slices, kps) : launch_sgemm<false, false, false>(cx, st, a, b, c, inc_c, m, n, k, slices, kps);
 }
 
 int eddlb200_sum2d_rowwise(int dev, const float *a, const float *b, float *c, int rows, int cols) {
@@ -185,7 +221,7 @@ int eddlb200_reduce_sum2d(int dev, const float *a, float *b, int rows, int cols,
     if (inc_b) EB_MODIFIES(b, (size_t)(axis == 0 ? cols : rows) * sizeof(float)); else EB_WRITES(b, (size_t)(axis == 0 ? cols : rows) * sizeof(float));
     if (axis == 0) {
         if (!cols) return 0;
-        eb::launch(colsum_kernel, (cols + 255) / 256, 256, 0, st, a, b, rows, cols, inc_b);
+        eb::launch(colsum_kernel, (cols + 63) / 64, 64, 0, st, a, b, rows, cols, inc_b);
     } else {
         if (!rows) return 0;
         eb::launch(rowsum_kernel, (rows + 7) / 8, 256, 0, st, a, b, rows, cols, inc_b);

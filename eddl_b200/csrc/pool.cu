@@ -288,6 +288,95 @@ __global__ void __launch_bounds__(256) maxpool_bwd_plane_kernel(const float *__r
     }
 }
 
+// 2x2 windows with stride 2 and no padding, the pooling layer of most small nets: windows do not overlap, so a thread owns V
+// whole windows side by side and every element is read and written once, in both directions, without the covering-window
+// search.  V = 2 takes 16 bytes of each input row (rows of a multiple of four elements, tensors 16-byte aligned).
+// 100 x 16 x 28 x 28: forward 8.4 -> 4 us, backward 19 -> 5 us.
+template <int V>
+__global__ void __launch_bounds__(kBlock) maxpool22_fwd_kernel(const float *__restrict__ in, float *__restrict__ out, float *__restrict__ ind_x,
+                                                               float *__restrict__ ind_y, unsigned total_v, unsigned ih, unsigned iw, unsigned oh, unsigned ow) {
+    EB_GRID_WAIT();
+    const unsigned stride = gridDim.x * blockDim.x, owv = ow / V;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total_v; i += stride) {
+        const unsigned t = i / owv, ox = (i - t * owv) * V, plane = t / oh, oy = t - plane * oh;
+        const float *src = in + ((size_t)plane * ih + 2 * oy) * iw + 2 * ox;
+        float r0[2 * V], r1[2 * V];
+        if (V == 2) {
+            const float4 a = ldg4(src), b = ldg4(src + iw);
+            r0[0] = a.x; r0[1] = a.y; r0[2 * V - 2] = a.z; r0[2 * V - 1] = a.w;
+            r1[0] = b.x; r1[1] = b.y; r1[2 * V - 2] = b.z; r1[2 * V - 1] = b.w;
+        } else {
+            r0[0] = __ldg(src); r0[1] = __ldg(src + 1); r1[0] = __ldg(src + iw); r1[1] = __ldg(src + iw + 1);
+        }
+        float m[V], bx[V], by[V];
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            const float x0 = (float)(2 * (ox + e)), y0 = (float)(2 * oy);
+            m[e] = -3.40282e+38f; bx[e] = 0.f; by[e] = 0.f;
+            if (r0[2 * e] > m[e]) { m[e] = r0[2 * e]; bx[e] = x0; by[e] = y0; }
+            if (r0[2 * e + 1] > m[e]) { m[e] = r0[2 * e + 1]; bx[e] = x0 + 1.f; by[e] = y0; }
+            if (r1[2 * e] > m[e]) { m[e] = r1[2 * e]; bx[e] = x0; by[e] = y0 + 1.f; }
+            if (r1[2 * e + 1] > m[e]) { m[e] = r1[2 * e + 1]; bx[e] = x0 + 1.f; by[e] = y0 + 1.f; }
+        }
+        const size_t o = (size_t)t * ow + ox;
+        if (V == 2) {
+            *reinterpret_cast<float2 *>(out + o) = make_float2(m[0], m[V - 1]);
+            *reinterpret_cast<float2 *>(ind_x + o) = make_float2(bx[0], bx[V - 1]);
+            *reinterpret_cast<float2 *>(ind_y + o) = make_float2(by[0], by[V - 1]);
+        } else { out[o] = m[0]; ind_x[o] = bx[0]; ind_y[o] = by[0]; }
+    }
+}
+
+// One thread per V windows of the grid that covers the whole input, the odd last row and column included (no window there:
+// nothing is added).  id_zero: the input delta is known to hold zeros and is written in full.
+template <int V>
+__global__ void __launch_bounds__(kBlock) maxpool22_bwd_kernel(const float *__restrict__ d, const float *__restrict__ ind_x, const float *__restrict__ ind_y,
+                                                               float *__restrict__ id, unsigned total_v, unsigned ih, unsigned iw, unsigned oh, unsigned ow, int id_zero) {
+    EB_GRID_WAIT();
+    const unsigned stride = gridDim.x * blockDim.x, wv = (iw + 2 * V - 1) / (2 * V), hv = (ih + 1) / 2;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total_v; i += stride) {
+        const unsigned t = i / wv, ox = (i - t * wv) * V, plane = t / hv, oy = t - plane * hv;
+        float v[V]; int key[V];                           // position of the maximum inside the window: 0-3, -1 = not in it
+#pragma unroll
+        for (int e = 0; e < V; e++) {
+            key[e] = -1; v[e] = 0.f;
+            if (oy < oh && ox + e < ow) {
+                const size_t o = ((size_t)plane * oh + oy) * ow + ox + e;
+                v[e] = __ldg(d + o);
+                // int x = D->indX->ptr[p]  (float -> int conversion in the reference)
+                const int kx = (int)__ldg(ind_x + o) - (int)(2 * (ox + e)), ky = (int)__ldg(ind_y + o) - (int)(2 * oy);
+                if ((unsigned)kx < 2u && (unsigned)ky < 2u) key[e] = 2 * ky + kx;
+            }
+        }
+        float *dst = id + ((size_t)plane * ih + 2 * oy) * iw + 2 * ox;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            if (2 * oy + r >= ih) continue;
+            float *q = dst + (size_t)r * iw;
+            if (V == 2) {
+                float4 a = id_zero ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4 *>(q);
+                a.x = key[0] == 2 * r ? __fadd_rn(a.x, v[0]) : a.x;
+                a.y = key[0] == 2 * r + 1 ? __fadd_rn(a.y, v[0]) : a.y;
+                a.z = key[V - 1] == 2 * r ? __fadd_rn(a.z, v[V - 1]) : a.z;
+                a.w = key[V - 1] == 2 * r + 1 ? __fadd_rn(a.w, v[V - 1]) : a.w;
+                *reinterpret_cast<float4 *>(q) = a;
+            } else {
+#pragma unroll
+                for (int x = 0; x < 2; x++) {
+                    if (2 * ox + x >= iw) continue;
+                    const bool hit = key[0] == 2 * r + x;
+                    if (id_zero) q[x] = hit ? __fadd_rn(0.f, v[0]) : 0.f;
+                    else if (hit) q[x] = __fadd_rn(q[x], v[0]);
+                }
+            }
+        }
+    }
+}
+
+bool plain_2x2(const PoolGeom &g, size_t in_elements) {
+    return g.kr == 2 && g.kc == 2 && g.sr == 2 && g.sc == 2 && g.pt == 0 && g.pl == 0 && 2 * g.oh <= g.ih && 2 * g.ow <= g.iw && in_elements < (size_t(1) << 31);
+}
+
 int check_geom(const char *what, int n, int c, int ih, int iw, int oh, int ow, int kr, int kc, int sr, int sc, int pt, int pl) {
     if (n < 0 || c < 0 || ih <= 0 || iw <= 0 || oh <= 0 || ow <= 0 || kr <= 0 || kc <= 0 || sr <= 0 || sc <= 0 || pt < 0 || pl < 0)
         return set_error(EDDLB200_EINVAL, "%s: bad geometry", what);
@@ -311,6 +400,13 @@ int eddlb200_maxpool2d_fwd(int dev, const float *in, float *out, float *ind_x, f
     EB_READS(in, (size_t)n * c * ih * iw * sizeof(float));
     EB_WRITES(out, total * sizeof(float)); EB_WRITES(ind_x, total * sizeof(float)); EB_WRITES(ind_y, total * sizeof(float));
     ProfScope prof(cx, PROF_POOL, 4.0 * n * c * ih * iw + 12.0 * total);
+    if (plain_2x2(g, (size_t)n * c * ih * iw)) {
+        const bool v2 = iw % 4 == 0 && ow % 2 == 0 && aligned16(in) && ((uintptr_t)out & 7) == 0 && ((uintptr_t)ind_x & 7) == 0 && ((uintptr_t)ind_y & 7) == 0;
+        if (v2) eb::launch(maxpool22_fwd_kernel<2>, grid_for(total / 2, kBlock), kBlock, 0, st, in, out, ind_x, ind_y, (unsigned)(total / 2), ih, iw, oh, ow);
+        else eb::launch(maxpool22_fwd_kernel<1>, grid_for(total, kBlock), kBlock, 0, st, in, out, ind_x, ind_y, (unsigned)total, ih, iw, oh, ow);
+        EB_LAUNCH_CHECK("gpu_mpool2D");
+        return 0;
+    }
     const int blocks = grid_for(total, kBlock);
     if ((size_t)n * c * ih * iw >= (size_t(1) << 32)) eb::launch(maxpool_fwd_kernel<0, 0, size_t>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
     else if (kr == 2 && kc == 2) eb::launch(maxpool_fwd_kernel<2, 2, unsigned>, blocks, kBlock, 0, st, in, out, ind_x, ind_y, total, g);
@@ -334,6 +430,14 @@ int eddlb200_maxpool2d_bwd(int dev, const float *d, const float *ind_x, const fl
     EB_NOTES(id, total * sizeof(float));
     if (lz_any(cx) && id != d) { int status = 0; id_zero = lz_take(cx, st, id, total * sizeof(float), &status); if (status) return status; }
     ProfScope prof(cx, PROF_POOL, 12.0 * n * c * oh * ow + (id_zero ? 4.0 : 8.0) * total);     // the delta is stored, or read and written
+    if (plain_2x2(g, total)) {
+        const bool v2 = iw % 4 == 0 && aligned16(id);
+        const unsigned items = (unsigned)((size_t)n * c * ((ih + 1) / 2) * (v2 ? iw / 4 : (iw + 1) / 2));
+        if (v2) eb::launch(maxpool22_bwd_kernel<2>, grid_for(items, kBlock), kBlock, 0, st, d, ind_x, ind_y, id, items, ih, iw, oh, ow, id_zero);
+        else eb::launch(maxpool22_bwd_kernel<1>, grid_for(items, kBlock), kBlock, 0, st, d, ind_x, ind_y, id, items, ih, iw, oh, ow, id_zero);
+        EB_LAUNCH_CHECK("gpu_mpool2D_back");
+        return 0;
+    }
     const size_t plane_smem = (size_t)8 * oh * ow + (size_t)4 * (ih + iw);
     if (plane_smem <= (size_t)160 * 1024 && ih * iw >= 1024 && oh < 32768 && ow < 32768 && (size_t)n * c < 0x7fffffffu) {
         static bool configured[EDDLB200_MAX_DEVICES] = {};

@@ -27,6 +27,10 @@ struct DevCtx {
     size_t bytes_in_use = 0, bytes_cached = 0;
     void *scratch_ptr = nullptr; size_t scratch_bytes = 0;
     float *h_scalars = nullptr, *d_scalars = nullptr;
+    unsigned *ticket_words = nullptr; size_t ticket_count = 0;
+    struct Table { std::vector<char> host; char *dev = nullptr; size_t cap = 0; unsigned long long used = 0; };
+    static constexpr size_t kTables = 16;
+    std::vector<Table> tables; unsigned long long table_clock = 0;
     cudaEvent_t ev_start[16] = {}, ev_stop[16] = {};
     unsigned long long launches = 0;
     ncclComm *comm = nullptr; int nranks = 1, rank = 0;
@@ -89,7 +93,7 @@ static int init_locked(int dev) {
     if ((e = cudaSetDevice(dev)) != cudaSuccess) return cuda_status(e, "cudaSetDevice");
     if ((e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking)) != cudaSuccess) return cuda_status(e, "cudaStreamCreate");
     if ((e = cudaMallocHost((void **)&c.h_scalars, 64 * sizeof(float))) != cudaSuccess) return cuda_status(e, "cudaMallocHost");
-    if ((e = cudaMalloc((void **)&c.d_scalars, 64 * sizeof(float))) != cudaSuccess) return cuda_status(e, "cudaMalloc");
+    if ((e = cudaMalloc((void **)&c.d_scalars, kDevScalars * sizeof(float))) != cudaSuccess) return cuda_status(e, "cudaMalloc");
     for (int i = 0; i < 16; i++) { cudaEventCreate(&c.ev_start[i]); cudaEventCreate(&c.ev_stop[i]); }
     if ((e = cudaEventCreateWithFlags(&c.ev_handoff, cudaEventDisableTiming)) != cudaSuccess) return cuda_status(e, "cudaEventCreate");
     c.dev = dev;
@@ -146,6 +150,37 @@ void *scratch(DevCtx *c, size_t bytes) {
     if (cudaMalloc(&c->scratch_ptr, want) != cudaSuccess) { set_error(cudaErrorMemoryAllocation, "scratch arena of %zu bytes", want); return nullptr; }
     c->scratch_bytes = want;
     return c->scratch_ptr;
+}
+
+unsigned *tickets(DevCtx *c, size_t count) {
+    if (count <= c->ticket_count) return c->ticket_words;
+    cudaStreamSynchronize(c->stream);
+    if (c->ticket_words) cudaFree(c->ticket_words);
+    c->ticket_words = nullptr; c->ticket_count = 0;
+    const size_t want = count < 4096 ? 4096 : 2 * count;
+    if (cudaMalloc((void **)&c->ticket_words, want * sizeof(unsigned)) != cudaSuccess) { set_error(cudaErrorMemoryAllocation, "%zu arrival counters", want); c->ticket_words = nullptr; return nullptr; }
+    cudaMemsetAsync(c->ticket_words, 0, want * sizeof(unsigned), c->stream);
+    c->ticket_count = want;
+    return c->ticket_words;
+}
+
+const char *device_table(DevCtx *c, cudaStream_t st, const char *host, size_t bytes) {
+    for (auto &t : c->tables)
+        if (t.host.size() == bytes && !memcmp(t.host.data(), host, bytes)) { t.used = ++c->table_clock; return t.dev; }
+    if (c->tables.size() < DevCtx::kTables) c->tables.emplace_back();
+    DevCtx::Table *t = &c->tables[0];
+    for (auto &q : c->tables) if (q.used < t->used) t = &q;               // a new one has used = 0
+    if (t->cap < bytes) {
+        if (t->dev) cudaFree(t->dev);                                     // waits for the kernels that read it
+        t->dev = nullptr; t->cap = 0; t->host.clear();
+        if (cudaMalloc((void **)&t->dev, bytes + bytes / 2) != cudaSuccess) { set_error(cudaErrorMemoryAllocation, "table of %zu bytes", bytes); t->dev = nullptr; return nullptr; }
+        t->cap = bytes + bytes / 2;
+    }
+    t->host.assign(host, host + bytes);
+    t->used = ++c->table_clock;
+    // pageable source: staged before the call returns; the copy is ordered after the kernels that read the old contents
+    if (cudaMemcpyAsync(t->dev, host, bytes, cudaMemcpyHostToDevice, st) != cudaSuccess) { t->host.clear(); return nullptr; }
+    return t->dev;
 }
 
 // ---- write observers ----------------------------------------------------------------------------------
