@@ -216,6 +216,7 @@ int eddlb200_set_option(const char *name, int value) {
     if (name && !strcmp(name, "lazy_zero") && (value == 0 || value == 1)) return lz_set_all(value);
     if (name && !strcmp(name, "conv_prefetch") && (value == 0 || value == 1)) return conv_tc_set_prefetch(value);
     if (name && !strcmp(name, "conv_tma") && value >= 0 && value <= 2) return conv_tc_set_tma(value);
+    if (name && !strcmp(name, "conv_pairs") && value >= 0 && value <= 2) return conv_tc_set_rs(value);
     if (name && !strcmp(name, "conv_pack_cache") && (value == 0 || value == 1)) return conv_tc_set_pack_cache(value);
     if (name && !strcmp(name, "conv_tma_3x3") && (value == 0 || value == 1)) return conv_tc_set_tma_3x3(value);
     if (name && !strcmp(name, "conv_dense_1x1") && (value == 0 || value == 1)) { g_conv_dense = value; return 0; }
@@ -245,6 +246,7 @@ int eddlb200_conv2d_fwd(int dev, const float *x, const float *w, const float *bi
     EB_WRITES(y, (size_t)n * k * oh * ow * sizeof(float));
     ProfScope prof(cx, PROF_CONV_FWD, 2.0 * n * (double)k * c * kr * kc * oh * ow);
     if (tc_enabled()) {
+        if (int r = conv_tc_rs(cx, st, 0, g, x, w, y, bias, precision, false); r != 1) { g_conv_calls[dev][0]++; return r; }
         const Dense1x1 d = dense_1x1(g, true);
         float *xs = d.on ? dense_buf(st, 0, (size_t)n * c * d.pitch * sizeof(float)) : nullptr;
         if (xs) {
@@ -274,6 +276,7 @@ int eddlb200_conv2d_bwd_data(int dev, const float *dy, const float *w, float *dx
     if (lz_any(cx)) { int status = 0; dx_zero = lz_take(cx, st, dx, dx_elems * sizeof(float), &status); if (status) return status; }
     ProfScope prof(cx, PROF_CONV_BWD_DATA, 2.0 * n * (double)k * c * kr * kc * oh * ow);
     if (tc_enabled()) {
+        if (int r = conv_tc_rs(cx, st, 1, g, dy, w, dx, nullptr, precision, dx_zero); r != 1) { g_conv_calls[dev][0]++; return r; }
         const Dense1x1 d = dense_1x1(g, true);
         float *dense = d.on ? dense_buf(st, 2, (size_t)n * c * d.pitch * sizeof(float)) : nullptr;
         if (dense) {

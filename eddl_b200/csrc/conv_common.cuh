@@ -26,6 +26,11 @@ int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const floa
 bool conv_tc_allowed();          // false while eddlb200_set_option("conv_path", 1) / EDDL_B200_CONV=simt forces the fp32 FMA kernels
 int conv_tc_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool gw_zero);
 
+// Forward (mode 0: src = x, out = y) and backward-data (mode 1: src = dy, out = dx) on pairs of CTAs (conv_rs.cuh); 1 = not taken.
+int conv_tc_rs(DevCtx *cx, cudaStream_t st, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias, int precision, bool out_zero);
+// 1 (default): that kernel runs the layers it is the faster one for; 2: every layer it fits; 0: none.
+int conv_tc_set_rs(int level);
+
 // 1 (default): the tensor-core kernel's prefetch warp pulls the activation operand of 1x1 layers into L2 ahead of the gather.
 int conv_tc_set_prefetch(int on);
 // 2 (default): 1x1 stride-1 forward / backward-data layers are fed and drained by TMA tensor copies, accumulating outputs by

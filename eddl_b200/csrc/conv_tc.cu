@@ -39,8 +39,7 @@
 // four whole rows; the tap-shifted x operand of larger filters keeps one lane per k.
 // Every wait on an mbarrier is bounded; on time-out the kernel records a status code, leaves
 // its loops, frees its tensor memory and returns.
-#include <cuda.h>
-#include <cuda_bf16.h>
+#include <algorithm>
 #include <array>
 #include <map>
 #include <mutex>
@@ -48,13 +47,13 @@
 #include <vector>
 #include "common.cuh"
 #include "conv_common.cuh"
+#include "tc_ptx.cuh"
+#include "conv_rs.cuh"
 
 namespace {
 
 using namespace eb;
 
-constexpr int BM = 128;             // UMMA M (TMEM lanes)
-constexpr int BK = 32;              // fp32 per 128-byte swizzle row
 constexpr int NPROD = 256;          // producer threads (warps 0-7); warp 8 issues the MMAs; warps 9-12 run the epilogue
 constexpr int NEPI = 128;           // epilogue threads (warps 9-12)
 constexpr int NTHREADS = NPROD + 32 + NEPI + 32;     // + warp 13: L2 prefetch of the activation operand / TMA issue
@@ -69,7 +68,6 @@ constexpr int WS_CH = 14, WS_ROWS = 9 * WS_CH, WS_SLAB_PX = 152, WS_SLAB_CH = 16
 constexpr int SLAB_PX = 256;        // pixels per channel of a raw slab (3x3 TMA-fed kernels): 128 rows + a halo of W + 1 either side + alignment
 constexpr int PF_AHEAD = 8;         // K-blocks the prefetch warp may run ahead of the producers
 constexpr int INVALID_Y = -20000;
-constexpr int NMAIN = 3;             // rotating hi*hi accumulators; a fourth holds the cross terms
 
 struct TcParams {
     const float *srcA, *srcB;
@@ -106,127 +104,6 @@ struct TcParams {
     alignas(64) CUtensorMap mapA;
     alignas(64) CUtensorMap mapOut;
 };
-
-// ---- PTX wrappers ---------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: gives up after ~2 s of SM clock, or as soon as another role of the CTA has given up (the abort flag), and
-// reports false.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 256; i++) if (mbar_try(bar, parity)) return true;
-        if (*abort_flag || clock64() - t0 > 4000000000LL) return false;
-    }
-}
-// The same for a whole warp: every lane waits, and the warp leaves together if any lane gave up, so that no warp-wide
-// (.sync.aligned, shuffle) instruction that follows is reached by part of a warp.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// TMA bulk copy global -> shared (1-D, 16-byte aligned, size a multiple of 16), completion counted on an mbarrier
-__device__ __forceinline__ void tma_bulk_g2s(uint32_t dst_smem, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-// TMA tensor copy global -> shared: a [1][32 channels][32 pixels] box of a 3-D tensor map; coordinates may lie outside the
-// tensor (the missing elements arrive as zeros), x must be a multiple of 4 elements
-__device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(dst_smem), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
-}
-// TMA tensor copy shared -> global (elements outside the tensor are dropped), plain store or fp32 add into global memory
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, int x, int y, int z, uint32_t src_smem) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];"
-                 ::"l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(src_smem) : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap *map, int x, int y, int z, uint32_t src_smem) {
-    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2, %3}], [%4];"
-                 ::"l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(src_smem) : "memory");
-}
-__device__ __forceinline__ void tma_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void tma_wait_group_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-template <int N> __device__ __forceinline__ void tma_wait_group() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// K-major SWIZZLE_128B shared-memory matrix descriptor: rows of 128 bytes, 8-row groups 1024 bytes
-// apart (stride byte offset), descriptor version 1, layout type 2, 1024-byte aligned tile base.
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-// fp32 accumulate, TF32 x TF32, both operands K-major, M = 128, N = bn
-__host__ __device__ constexpr uint32_t make_idesc(int bn) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-
-// fp32 accumulate, BF16 x BF16 (kind::f16), both operands K-major, M = 128, N = bn, K = 16 per instruction
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int bn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-}
-
-// byte offset of 16-byte chunk `chunk` of row `row` inside a [rows][128 bytes] SWIZZLE_128B tile
-__device__ __forceinline__ uint32_t swz_chunk(uint32_t row, uint32_t chunk) { return row * 128u + (((chunk ^ row) & 7u) << 4); }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);          // a in the low half = the lower address
-    return *reinterpret_cast<const uint32_t *>(&v);
-}
-
-__device__ __forceinline__ void split_tf32(float v, float &hi, float &lo) {
-    hi = __uint_as_float(__float_as_uint(v) & 0xFFFFE000u);
-    lo = __fsub_rn(v, hi);
-}
-
-// byte offset of element (row, k) inside a [rows][32 fp32] SWIZZLE_128B tile
-__device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t k) {
-    return row * 128u + ((((k >> 2) ^ row) & 7u) << 4) + ((k & 3u) << 2);
-}
 
 // Shared memory of a CTA.  Gather kernels: the operand ring only.  ATMA kernels add a ring of RAW_STAGES raw activation
 // tiles ([4 chunks][32 channels][32 pixels] fp32, written by TMA) in front of the converters and two 4 KB staging buffers
@@ -825,31 +702,38 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
         }
     } else if (warp == 8) {
         // ============================ MMA issuer (one thread) ============================
-        // One thread feeds the tensor core, so its instruction stream is kept short: shared-memory descriptors differ only
-        // in their 14-bit address field, which is advanced by adding constants (no field of the low word can carry into the
-        // next: shared addresses stay below 256 KB), and stage / phase / accumulator rotation are running counters.
-        if (lane == 0) {
+        // One thread feeds the tensor core, and the queue between the two is shallow: an MMA of 128 columns runs for 64 cycles, and
+        // whatever takes the thread longer than that between two of them is time the tensor pipe stands still.  So nothing in the
+        // loop waits for a result: shared-memory descriptors differ only in their 14-bit address field, which is advanced by
+        // adding constants (no field of the low word can carry into the next: shared addresses stay below 256 KB); the rotation
+        // over the main accumulators is a renaming of three registers; and the barrier of the NEXT stage is looked at in the
+        // middle of a K-block, so that its answer is there when the K-block has been issued.  A loop that issues 12 MMAs and then
+        // waits for the next stage takes 1017 cycles per K-block with every operand ready, this one 800 (768 are the MMAs).
+        if (elect_one()) {
             const uint32_t idesc = make_idesc(BN_);
             constexpr uint32_t DESC_HI = 64u | (1u << 14) | (2u << 29);       // upper word of make_desc()
             auto desc = [&](uint32_t lo) { return ((uint64_t)DESC_HI << 32) | lo; };
             const uint32_t stage0_lo = ((smem_u32(stage_base) >> 4) & 0x3FFFu) | (1u << 16);
             constexpr uint32_t STAGE_STEP = (uint32_t)L::STAGE_BYTES >> 4, A_STEP = (uint32_t)L::A_BYTES >> 4, B_STEP = (uint32_t)L::B_BYTES >> 4;
-            int local = 0, set = 0;
-            uint32_t s = 0, full_phase = 0, set_phase = 1, wh = 0;
+            constexpr uint32_t RING = WMODE ? 2u : (uint32_t)STAGES;
+            int set = 0;
+            uint32_t s = 0, full_phase = 0, set_phase = 1, wh = 0, ready = 0;
             auto lo_word = [&](const uint8_t *ptr) { return ((smem_u32(ptr) >> 4) & 0x3FFFu) | (1u << 16); };
             const uint32_t w_hib_lo = lo_word(w_hib), w_lo_lo = lo_word(w_lo), w_x_lo = lo_word(w_x);
             const int nmain = P.nmain;
-            for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x, local++) {
+            const uint32_t rot_step = nmain > 1 ? (uint32_t)BN_ : 0u;
+            for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x) {
                 int kb0, nkb; kb_range(t, kb0, nkb);
                 if (!mbar_wait(bar_acc_empty + 8 * set, set_phase, abort_flag)) { failed = true, fail_code = 10; break; }
                 tc_fence_after();
                 const uint32_t set_base = tmem_base + (uint32_t)(set * set_cols);
                 const uint32_t d_small = set_base + (uint32_t)small_off;
-                int rot = 0;                   // which of the rotating main accumulators the next k-step adds into
-                int fresh = nmain + 1;         // accumulators not written yet in this tile: the mains' first k-steps and the cross terms' first
+                // the main accumulators of this K-block's k-steps: d0, d1, d2, d0; the next K-block starts with d1
+                uint32_t d0 = set_base, d1 = set_base + rot_step, d2 = d1 + rot_step;
                 for (int it = 0; it < nkb; it++) {
-                    if (!mbar_wait(bar_full + 8 * s, full_phase, abort_flag)) { failed = true, fail_code = 11; break; }
+                    if (!ready && !mbar_wait(bar_full + 8 * s, full_phase, abort_flag)) { failed = true, fail_code = 11; break; }
                     tc_fence_after();
+                    const uint32_t next_s = s + 1 == RING ? 0u : s + 1, next_phase = full_phase ^ (s + 1 == RING ? 1u : 0u);
                     uint32_t a_hi = stage0_lo + s * STAGE_STEP;
                     uint32_t a_lo = a_hi + A_STEP;
                     uint32_t b_hi = a_hi + (SPLIT3 ? 2u : 1u) * A_STEP;
@@ -861,29 +745,31 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
                         if constexpr (WTMA) { a_hi = w_x_lo + wh * A_STEP; a_lo = lo_slot; b_lo = lo_slot + A_STEP; }
                         else { a_hi = lo_slot; a_lo = lo_slot + A_STEP; b_lo = lo_slot + (SPLIT3 ? 2u : 1u) * A_STEP; }
                     }
+                    // an accumulator's first k-step in a tile overwrites it
+                    const uint32_t old0 = it ? 1u : 0u, old12 = it || nmain == 1 ? 1u : 0u;
 #pragma unroll
                     for (int ks = 0; ks < BK / 8; ks++) {
                         const uint32_t o = 2u * ks;      // 8 fp32 = 32 bytes along K inside the swizzle row = 2 units of 16 bytes
-                        const bool first = (it == 0 && ks == 0);
                         if (SPLIT3) {
                             if (!CROSS_BF16) {
-                                umma_tf32(d_small, desc(a_lo + o), desc(b_hi + o), idesc, first ? 0u : 1u);
+                                umma_tf32(d_small, desc(a_lo + o), desc(b_hi + o), idesc, ks ? 1u : old0);
                                 umma_tf32(d_small, desc(a_hi + o), desc(b_lo + o), idesc, 1u);
                             } else {
                                 // cross terms in bf16: 16 of the 64 [lo | hi] x [hi | lo] columns per instruction
-                                umma_bf16(d_small, desc(a_lo + o), desc(b_lo + o), make_idesc_bf16(BN_), first ? 0u : 1u);
+                                umma_bf16(d_small, desc(a_lo + o), desc(b_lo + o), make_idesc_bf16(BN_), ks ? 1u : old0);
                             }
                         }
-                        umma_tf32(set_base + (uint32_t)(rot * BN_), desc(a_hi + o), desc(b_hi + o), idesc, fresh > 1 ? 0u : 1u);
-                        if (fresh > 1) fresh--;
-                        if (++rot == nmain) rot = 0;
+                        umma_tf32(ks == 1 ? d1 : ks == 2 ? d2 : d0, desc(a_hi + o), desc(b_hi + o), idesc, ks == 0 ? old0 : ks == 3 ? 1u : old12);
+                        if (ks == 1) ready = mbar_test(bar_full + 8 * next_s, next_phase);
                     }
                     umma_commit(bar_empty + 8 * s);      // frees the stage (WMODE: the LO slot) when these MMAs have read it
                     if constexpr (WMODE) {
                         umma_commit(bar_raw_full + 8 * (HS + wh));      // ... and the HI slot
                         if (++wh == (uint32_t)HS) wh = 0;
-                        if (++s == 2u) { s = 0; full_phase ^= 1u; }
-                    } else if (++s == (uint32_t)STAGES) { s = 0; full_phase ^= 1u; }
+                    }
+                    s = next_s; full_phase = next_phase;
+                    const uint32_t first = d0;
+                    d0 = d1; d1 = d2; d2 = first;
                 }
                 if (!failed) umma_commit(bar_acc_full + 8 * set);     // this tile's accumulators are complete
                 if (++set == nsets) { set = 0; set_phase ^= 1u; }
@@ -1248,6 +1134,40 @@ __global__ void __launch_bounds__(256) build_tables_kernel(TableArgs T) {
             }
         } else if (i < (long long)T.M_total + T.K_pad) {
             const int k = (int)(i - T.M_total);
+            if (T.check == 7) {
+                // row-shift kernels: k = (class, 32-channel group, tap of the class, channel in group); only the weight offsets are needed
+                const int nch = T.mode == 0 ? g.c : g.k, cgs = (nch + BK - 1) / BK, ch_in = k & (BK - 1);
+                int kb = k / BK, r = 0, s = 0;
+                if (T.mode == 0) {
+                    // taps in the order of the input phases they read: (row parity, column parity), then row by row
+                    int t = kb % rs;
+                    kb /= rs;
+                    for (int rho = 0, found = 0; rho < g.sr && !found; rho++)
+                        for (int sig = 0; sig < g.sc && !found; sig++)
+                            for (r = 0; r < g.kr && !found; r++) {
+                                if (((r - g.pt) % g.sr + g.sr) % g.sr != rho) continue;
+                                for (s = 0; s < g.kc && !found; s++)
+                                    if (((s - g.pl) % g.sc + g.sc) % g.sc == sig && t-- == 0) found = 1;
+                            }
+                    r--; s--;                       // the loops step once more on their way out
+                } else {
+                    for (int ca = 0, found = 0; ca < g.sr && !found; ca++)
+                        for (int cb = 0; cb < g.sc && !found; cb++) {
+                            const int y0 = ((ca - g.pt) % g.sr + g.sr) % g.sr, x0 = ((cb - g.pl) % g.sc + g.sc) % g.sc;
+                            const int rt = ca < g.kr ? (g.kr - ca + g.sr - 1) / g.sr : 0, st = cb < g.kc ? (g.kc - cb + g.sc - 1) / g.sc : 0;
+                            if (rt * st == 0 || y0 >= g.ih || x0 >= g.iw) continue;
+                            if (kb >= cgs * rt * st) { kb -= cgs * rt * st; continue; }
+                            const int t = kb % (rt * st);
+                            kb /= rt * st;
+                            r = ca + (t / st) * g.sr; s = cb + (t % st) * g.sc;
+                            found = 1;
+                        }
+                }
+                const int ch = kb * BK + ch_in;
+                T.kA[k] = make_int2(0, 0); T.kC[k] = 0;
+                T.kB[k] = ch >= nch ? -1 : (T.mode == 0 ? ch * rs + r * g.kc + s : ch * g.c * rs + r * g.kc + s);
+                continue;
+            }
             if (T.check == 5) {
                 // slab-fed 3x3 kernels: k = (32-channel group, tap, channel in group); only the weight offsets are needed
                 const int cg = k / (9 * BK), rem = k - cg * 9 * BK, tap = rem / BK, ch = cg * BK + (rem - tap * BK);
@@ -1399,17 +1319,10 @@ int launch_bn(DevCtx *cx, cudaStream_t st, const TcParams &P, dim3 grid, int bn,
     return launch_variant<128, PREC, WGRAD, BGATHER, TMA>(cx, st, P, grid, dev);
 }
 
-// [images][channels][pixels] fp32 tensor as a 3-D tensor map with boxes of 32 pixels x 32 channels of one image, no swizzle:
-// the box lands in shared memory as [32 channels][32 pixels].  Needs a 16-byte aligned base and pixels % 4 == 0.
-// With swizzle128 the box (box_rows channels x 32 pixels = box_rows rows of 128 bytes) lands in the K-major SWIZZLE_128B layout
-// of an MMA operand whose k runs along the pixels.
-bool encode_plane_map(CUtensorMap *map, const float *base, int pixels, int channels, int images, int box_rows = 32, bool swizzle128 = false, int box_px = 32) {
-    const cuuint64_t dims[3] = {(cuuint64_t)pixels, (cuuint64_t)channels, (cuuint64_t)images};
-    const cuuint64_t strides[2] = {(cuuint64_t)pixels * 4, (cuuint64_t)pixels * channels * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)box_px, (cuuint32_t)box_rows, 1}, elem[3] = {1, 1, 1};
-    // the driver entry point is looked up at run time: the library must load (and refuse work) on a machine without a driver
-    typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// the driver entry point is looked up at run time: the library must load (and refuse work) on a machine without a driver
+typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                             const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn encode_function() {
     static EncodeFn encode = nullptr;
     static bool looked_up = false;
     if (!looked_up) {
@@ -1419,6 +1332,18 @@ bool encode_plane_map(CUtensorMap *map, const float *base, int pixels, int chann
         else cudaGetLastError();
         looked_up = true;
     }
+    return encode;
+}
+
+// [images][channels][pixels] fp32 tensor as a 3-D tensor map with boxes of 32 pixels x 32 channels of one image, no swizzle:
+// the box lands in shared memory as [32 channels][32 pixels].  Needs a 16-byte aligned base and pixels % 4 == 0.
+// With swizzle128 the box (box_rows channels x 32 pixels = box_rows rows of 128 bytes) lands in the K-major SWIZZLE_128B layout
+// of an MMA operand whose k runs along the pixels.
+bool encode_plane_map(CUtensorMap *map, const float *base, int pixels, int channels, int images, int box_rows = 32, bool swizzle128 = false, int box_px = 32) {
+    const cuuint64_t dims[3] = {(cuuint64_t)pixels, (cuuint64_t)channels, (cuuint64_t)images};
+    const cuuint64_t strides[2] = {(cuuint64_t)pixels * 4, (cuuint64_t)pixels * channels * 4};
+    const cuuint32_t box[3] = {(cuuint32_t)box_px, (cuuint32_t)box_rows, 1}, elem[3] = {1, 1, 1};
+    const EncodeFn encode = encode_function();
     if (!encode) return false;
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, elem,
                                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1430,6 +1355,12 @@ int g_conv_wslab = 1;          // eddlb200_set_option("conv_tma_wgrad_3x3", 0 / 
 int g_conv_wtma = 2;           // eddlb200_set_option("conv_tma_wgrad", 0 off / 1 on / 2 on, landed values used as the hi plane as they are)
 
 int *g_status[EDDLB200_MAX_DEVICES] = {};
+int status_word(int dev, cudaStream_t st) {
+    if (g_status[dev]) return 0;
+    if (cudaMalloc((void **)&g_status[dev], sizeof(int)) != cudaSuccess) return cudaErrorMemoryAllocation;
+    cudaMemsetAsync(g_status[dev], 0, sizeof(int), st);
+    return 0;
+}
 int g_conv_prefetch = 1;       // eddlb200_set_option("conv_prefetch", 0 / 1)
 
 // The index tables are a pure function of the problem geometry, so they are built once per distinct geometry and kept
@@ -1449,10 +1380,24 @@ std::array<int, 24> table_key(const TableArgs &T) {
             T.ca, T.cb, T.y0, T.x0, T.hc, T.wc, T.rt, T.st_, T.check, T.K_pad};
 }
 
+// Device memory for the tables of `key`, kept across calls (build = they have yet to be written); nullptr past the budget.
+char *cached_table(int dev, const std::array<int, 24> &key, size_t bytes, bool &build) {
+    TableCache &tc = g_tables[dev];
+    std::lock_guard<std::mutex> lock(tc.mu);
+    build = true;
+    auto it = tc.entries.find(key);
+    if (it != tc.entries.end()) { build = false; return it->second; }
+    char *tb = nullptr;
+    if (tc.bytes + bytes > kTableCacheBudget || cudaMalloc((void **)&tb, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    tc.entries.emplace(key, tb); tc.bytes += bytes;
+    return tb;
+}
+
 // Packed weight images, one per (weight tensor, tiling), valid while the tensor's write-observer version stands.
 struct PackEntry {
     std::array<int, 24> tkey; int bn, precision; const float *src; size_t src_bytes;
     float *packed; size_t packed_bytes;
+    CUtensorMap map; bool has_map;         // the image as rows of 32 floats (row-shift kernels)
     unsigned blocks;                       // K-blocks x filter tiles = thread blocks that pack it
     unsigned long long version;            // version of src the image was made from (0 = never)
 };
@@ -1467,7 +1412,7 @@ int g_conv_pack_cache = 1;                 // eddlb200_set_option("conv_pack_cac
 // The packed image of `src` for this tiling, re-packing every out-of-date image of the device in one launch when this
 // one is out of date.  nullptr = not cached (the caller packs into scratch for this call).  rowB / kB must be cached tables.
 const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::array<int, 24> &tkey, int bn, int precision, const float *src,
-                            size_t src_bytes, const int *rowB, const int *kB, int kblocks, int tiles_n, int n_total, int row_fastest) {
+                            size_t src_bytes, const int *rowB, const int *kB, int kblocks, int tiles_n, int n_total, int row_fastest, PackEntry **entry = nullptr) {
     if (!g_conv_pack_cache) return nullptr;
     PackCache &pc = g_packs[dev];
     std::lock_guard<std::mutex> lock(pc.mu);
@@ -1497,6 +1442,7 @@ const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::arr
         }
         PackEntry &e = pc.entries[slot];
         if (!e.packed && cudaMalloc((void **)&e.packed, packed_bytes) != cudaSuccess) { cudaGetLastError(); e = PackEntry{}; return nullptr; }
+        e.has_map = false;
         e.tkey = tkey; e.bn = bn; e.precision = precision; e.src = src; e.src_bytes = src_bytes; e.packed_bytes = packed_bytes;
         e.blocks = (unsigned)kblocks * (unsigned)tiles_n; e.version = 0;
         const PackJob job{src, rowB, kB, e.packed, bn, n_total, tiles_n, row_fastest, precision, kblocks};
@@ -1505,6 +1451,7 @@ const float *packed_weights(DevCtx *cx, cudaStream_t st, int dev, const std::arr
     }
     PackEntry &me = pc.entries[slot];
     const unsigned long long now = watch_add(cx, src, src_bytes);         // registers the tensor on first use
+    if (entry) *entry = &me;
     if (me.version != 0 && me.version == now) return me.packed;
     // out of date: this image and every other one whose tensor has been written since it was packed
     MultiPackArgs A;
@@ -1537,6 +1484,257 @@ __global__ void __launch_bounds__(256) splitk_store_kernel(const float *__restri
         if (bias) v = __fadd_rn(v, __ldg(bias + (i / plane) % nbias));
         out[i] = v;
     }
+}
+
+// The packed weight image as a matrix of 128-byte rows with boxes of box_rows rows.
+bool encode_rows_map(CUtensorMap *map, const float *base, size_t rows, int box_rows) {
+    const cuuint64_t dims[2] = {32, (cuuint64_t)rows}, strides[1] = {128};
+    const cuuint32_t box[2] = {32, (cuuint32_t)box_rows}, elem[2] = {1, 1};
+    const EncodeFn encode = encode_function();
+    return encode && encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int BN_, int PREC>
+int launch_rs(DevCtx *cx, cudaStream_t st, const RsParams &P, int grid, int smem, int dev) {
+    static int configured_dev[EDDLB200_MAX_DEVICES] = {};
+    if (configured_dev[dev] < smem) {
+        cudaError_t e = cudaFuncSetAttribute(conv_rs_kernel<BN_, PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_LIMIT);
+        if (e != cudaSuccess) return cuda_status(e, "conv_rs(smem attribute)");
+        configured_dev[dev] = RS_SMEM_LIMIT;
+    }
+    eb::launch(conv_rs_kernel<BN_, PREC>, grid, RS_THREADS, smem, st, P);
+    EB_LAUNCH_CHECK("conv_rs");
+    if (P.splits > 1) {
+        eb::launch(rs_combine_kernel<BN_>, dim3(2 * P.ncls * P.tiles_m * P.tiles_n, BN_ / 8), 256, 0, st, P);
+        EB_LAUNCH_CHECK("conv_rs(combine)");
+    }
+    return 0;
+}
+template <int PREC>
+int launch_rs_bn(DevCtx *cx, cudaStream_t st, const RsParams &P, int grid, int smem, int bn, int dev) {
+    if (bn == 32) return launch_rs<32, PREC>(cx, st, P, grid, smem, dev);
+    if (bn == 64) return launch_rs<64, PREC>(cx, st, P, grid, smem, dev);
+    return launch_rs<128, PREC>(cx, st, P, grid, smem, dev);
+}
+
+// ---- which kernel: estimates in microseconds, calibrated on the layers of the nets at batch 1 to 128 ----
+constexpr int kMaxChainBlocks = 160;       // K-blocks per split: see the accumulator drift in run_one
+struct SplitChoice { int splits; double us; };
+// Split the reduction of `tiles` output tiles over the SMs: the makespan of `tiles * splits` work items dealt round-robin is
+// ceil(items / SMs) rounds of (K-blocks per split + one epilogue); splitting also costs a write and a read of every partial output.
+SplitChoice pick_splits(long long tiles, int kblocks, double t_kblock, size_t out_total, int sp_min) {
+    const double t_epilogue = 3.0;
+    int max_splits = kblocks / 4 < 128 ? kblocks / 4 : 128;
+    if (max_splits < sp_min) max_splits = sp_min + sp_min / 4;
+    SplitChoice best{sp_min, 1e30};
+    for (int sp = sp_min; sp <= max_splits; sp++) {
+        const int kb = (kblocks + sp - 1) / sp;
+        if ((kblocks + kb - 1) / kb != sp) continue;
+        const long long rounds = (tiles * sp + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS;
+        double cost = (double)rounds * (kb * t_kblock + t_epilogue);
+        if (sp > 1) cost += 3.0 + 2.0 * (double)out_total * sizeof(float) * sp / 6.0e6;
+        if (cost < best.us * 0.97) best = SplitChoice{sp, cost};          // prefer fewer splits unless the gain is clear
+    }
+    if (best.us >= 1e30) best.us = (double)((tiles * sp_min + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS) * ((double)kblocks / sp_min * t_kblock + t_epilogue);
+    return best;
+}
+inline int tile_n(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : 128); }
+inline double gather_us(int bn) { return bn == 128 ? 1.0 : bn == 64 ? 0.85 : 0.75; }          // one K-block of the gather kernel
+// the TMA-fed kernels: 0.62 us per K-block, no split
+inline double tma_fed_us(long long tiles, int kblocks) { return (double)((tiles + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS) * (kblocks * 0.62 + 1.2) + 2.5; }
+// forward / backward-data of a stride-1 layer on the gather kernel, with the splits it would choose
+double gather_layer_us(const ConvGeom &g, int mode) {
+    const int N = mode == 0 ? g.k : g.c, bn = tile_n(N);
+    const long long M = (long long)g.n * (mode == 0 ? g.oh * g.ow : g.ih * g.iw);
+    const int kblocks = ((mode == 0 ? g.c : g.k) * g.kr * g.kc + BK - 1) / BK;
+    return pick_splits((M + BM - 1) / BM * ((N + bn - 1) / bn), kblocks, gather_us(bn), (size_t)M * N, (kblocks + kMaxChainBlocks - 1) / kMaxChainBlocks).us;
+}
+
+// What the row-shift kernel would do with a layer: the padded position space, slabs and classes (see conv_rs.cuh), tile width and
+// number of splits.  false = the layer does not fit it.
+struct RsPlan { RsParams P; int bn, smem, kblocks; double us; };
+bool conv_rs_plan(const ConvGeom &g, int mode, int precision, RsPlan &plan) {
+    RsParams &P = plan.P;
+    P = RsParams{};
+    const int planes = precision == 1 ? 1 : 2;
+    struct Tap { int a, b; };
+    std::vector<Tap> taps;
+    int H0 = 0, W0 = 0, amin = 0, amax = 0, bmin = 0, bmax = 0, dh = 0, dw = 0;
+    if ((long long)g.kr * g.kc > RS_MAX_TAPS || g.sr * g.sc > RS_MAX_SLABS) return false;
+    auto fmod_ = [](int v, int m) { return ((v % m) + m) % m; };
+    int nslab = 0;
+    if (mode == 0) {
+        P.C = g.c; P.sh = g.ih; P.sw = g.iw; P.ssr = g.sr; P.ssc = g.sc; P.K = g.k; P.dhw = g.oh * g.ow; P.dw_full = g.ow; P.dsr = P.dsc = 1;
+        dh = g.oh; dw = g.ow;
+        for (int rho = 0; rho < g.sr; rho++)
+            for (int sig = 0; sig < g.sc; sig++) {
+                RsSlab &s = P.slab[nslab];
+                s.tap0 = (int)taps.size(); s.rho = rho; s.sigma = sig;
+                for (int r = 0; r < g.kr; r++)
+                    for (int q = 0; q < g.kc; q++)
+                        if (fmod_(r - g.pt, g.sr) == rho && fmod_(q - g.pl, g.sc) == sig) taps.push_back({(r - g.pt - rho) / g.sr, (q - g.pl - sig) / g.sc});
+                s.ntaps = (int)taps.size() - s.tap0;
+                if (!s.ntaps) continue;
+                H0 = std::max(H0, (g.ih - rho + g.sr - 1) / g.sr); W0 = std::max(W0, (g.iw - sig + g.sc - 1) / g.sc);
+                nslab++;
+            }
+        P.ncls = 1;
+        P.cls[0] = RsClass{0, nslab, (int)taps.size(), 0, g.oh, g.ow, 0, 0};
+    } else {
+        P.C = g.k; P.sh = g.oh; P.sw = g.ow; P.ssr = P.ssc = 1; P.K = g.c; P.dhw = g.ih * g.iw; P.dw_full = g.iw; P.dsr = g.sr; P.dsc = g.sc;
+        H0 = g.oh; W0 = g.ow;
+        int kb = 0;
+        for (int ca = 0; ca < g.sr; ca++)
+            for (int cb = 0; cb < g.sc; cb++) {
+                const int y0 = fmod_(ca - g.pt, g.sr), x0 = fmod_(cb - g.pl, g.sc);
+                const int rt = ca < g.kr ? (g.kr - ca + g.sr - 1) / g.sr : 0, sq = cb < g.kc ? (g.kc - cb + g.sc - 1) / g.sc : 0;
+                if (rt * sq == 0 || y0 >= g.ih || x0 >= g.iw) continue;              // this class receives nothing
+                const int cy = (y0 + g.pt - ca) / g.sr, cx = (x0 + g.pl - cb) / g.sc;
+                P.slab[nslab] = RsSlab{0, 0, (int)taps.size(), rt * sq, 0, 0};
+                for (int r = 0; r < rt; r++) for (int q = 0; q < sq; q++) taps.push_back({cy - r, cx - q});
+                RsClass &c = P.cls[P.ncls++];
+                c = RsClass{nslab, 1, rt * sq, kb, (g.ih - y0 + g.sr - 1) / g.sr, (g.iw - x0 + g.sc - 1) / g.sc, y0, x0};
+                dh = std::max(dh, c.dh); dw = std::max(dw, c.dw);
+                kb += rt * sq * ((P.C + BK - 1) / BK);
+                nslab++;
+            }
+    }
+    if (taps.empty()) return false;
+    for (const Tap &t : taps) { amin = std::min(amin, t.a); amax = std::max(amax, t.a); bmin = std::min(bmin, t.b); bmax = std::max(bmax, t.b); }
+    // a shift that leaves the image must land in the padding: rows as wide as the image plus the larger overhang (the left
+    // overhang of a row is the right overhang of the row before it), likewise the images
+    P.Wp = std::max(W0 + std::max({-bmin, dw + bmax - W0, 0}), dw);
+    const int Hp = std::max(H0 + std::max({-amin, dh + amax - H0, 0}), dh);
+    const long long positions = (long long)g.n * Hp * P.Wp;
+    if (positions > 0x7fffffffLL - 4096 || (long long)amax * P.Wp + bmax > 4096 || (long long)-amin * P.Wp - bmin > 4096) return false;
+    P.img_pos = Hp * P.Wp; P.images = g.n; P.M_total = (int)positions;
+    int rows = 0;
+    for (int i = 0; i < nslab; i++) {
+        RsSlab &s = P.slab[i];
+        int lo = 1 << 30, hi = -(1 << 30);
+        for (int t = s.tap0; t < s.tap0 + s.ntaps; t++) { const int sh = taps[t].a * P.Wp + taps[t].b; lo = std::min(lo, sh); hi = std::max(hi, sh); }
+        s.min_shift = lo; s.rows = 128 + hi - lo;
+        for (int t = s.tap0; t < s.tap0 + s.ntaps; t++) P.tap_row[t] = (short)(taps[t].a * P.Wp + taps[t].b - lo);
+        rows = std::max(rows, s.rows);
+    }
+    P.cgs = (P.C + BK - 1) / BK;
+    P.slab_plane = (rows + 7) / 8 * 1024;
+    plan.kblocks = P.cgs * (int)taps.size();
+    P.tiles_m = (int)((positions + 255) / 256);
+    // Tile width and splits by an estimate of the makespan in microseconds: rounds of tiles over the 74 pairs.  A tile's slab takes
+    // its taps' K-blocks (0.47 us at 128 filters; below that the MMAs' operand reads do not shrink with the tile) or its own
+    // conversion, whichever is longer, plus the drain; splitting adds the partial sums' way through memory and a launch.
+    const double c_kb[3] = {precision == 1 ? 0.20 : 0.31, precision == 1 ? 0.22 : 0.36, precision == 0 ? 0.47 : precision == 1 ? 0.27 : 0.36};
+    int min_kb = 1 << 30, max_kb = 0, max_taps = 1;
+    for (int c = 0; c < P.ncls; c++) { min_kb = std::min(min_kb, P.cls[c].taps * P.cgs); max_kb = std::max(max_kb, P.cls[c].taps * P.cgs); max_taps = std::max(max_taps, P.cls[c].taps); }
+    const double slab_us = 1.1 * ((rows + 127) / 128) * (P.ssc > 1 ? 1.8 : 1.0);
+    plan.us = 1e30;
+    for (int i = 0; i < 3; i++) {
+        const int bn = 32 << i, fixed = 2048 + planes * (bn / 2) * 128 * 2;
+        if (i > 0 && P.K <= bn / 2) continue;
+        if (2 * planes * P.slab_plane + fixed + RS_BAR_WORDS * 8 > RS_SMEM_LIMIT) continue;
+        const int tiles_n = (P.K + bn - 1) / bn;
+        const long long items = (long long)P.tiles_m * tiles_n;          // per class
+        if (items * P.ncls > (1 << 28)) continue;
+        double group = 0;                                                // one channel group of every class
+        for (int q = 0; q < nslab; q++) group += std::max(P.slab[q].ntaps * c_kb[i], slab_us);
+        for (int sp = 1; sp <= 64 && sp <= min_kb; sp++) {
+            if ((max_kb + sp - 1) / sp > kMaxChainBlocks && sp < min_kb) continue;          // accumulation chains stay short (see run_one)
+            const double rounds = (double)((items * P.ncls * sp + 73) / 74) / P.ncls;
+            double us = 4.0 + rounds * (std::max(group * P.cgs / sp, slab_us) + (i == 2 ? 2.6 : 1.3) * P.ncls);
+            if (sp > 1) us += 4.5 + (double)items * P.ncls * sp * bn * 256 * 8 / 5.0e6;
+            if (us < plan.us * 0.98) { plan.us = us; plan.bn = bn; P.splits = sp; }
+        }
+    }
+    if (plan.us >= 1e30) return false;
+    P.tiles_n = (P.K + plan.bn - 1) / plan.bn;
+    const int stage = planes * (plan.bn / 2) * 128, budget = RS_SMEM_LIMIT - 1024 - RS_BAR_WORDS * 8 - 64;
+    P.nbuf = 2;
+    while (P.nbuf < RS_MAX_BUF && (P.nbuf + 1) * planes * P.slab_plane + 4 * stage <= budget) P.nbuf++;
+    P.bst = std::min(RS_MAX_BST, (budget - P.nbuf * planes * P.slab_plane) / stage);
+    if (P.bst < 2) return false;
+    plan.smem = 1024 + P.nbuf * planes * P.slab_plane + P.bst * stage + RS_BAR_WORDS * 8 + 64;
+    const int chain = ((max_kb + P.splits - 1) / P.splits) * (std::min(P.C, BK) + 7) / 8;
+    P.nmain = chain > 64 ? NMAIN : 1;
+    return true;
+}
+
+int g_conv_rs = 1;             // eddlb200_set_option("conv_pairs", 0 off / 1 where it is the faster kernel / 2 wherever it fits)
+
+// mode 0 forward, 1 backward-data; 1 = not taken
+int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias,
+           int precision, bool out_zero) {
+    if (!g_conv_rs) return 1;
+    RsPlan plan;
+    if (!conv_rs_plan(g, mode, precision, plan)) return 1;
+    RsParams &P = plan.P;
+    if (g_conv_rs < 2) {
+        // Layers of a few channels stay on the gather kernels (a K-block here is 32 channels of one tap), layers of a few dx channels
+        // with their GEMM route; otherwise the smaller estimate wins.
+        if (P.C < 16 || P.K < 8 || (mode == 1 && g.c <= 8)) return 1;
+        const bool dense = g.sr == 1 && g.sc == 1;
+        double other = gather_layer_us(g, mode);
+        if (mode == 1 && !dense) other *= 2.0;                            // one launch per parity class, none of them split
+        const int bn = tile_n(P.K), tiles_n = (P.K + bn - 1) / bn, pq = g.oh * g.ow;
+        if (g.kr == 1 && g.kc == 1 && g.pt == 0 && g.pl == 0 && P.C >= 32 && P.K >= 32 && pq >= 32)
+            other = std::min(other, tma_fed_us(((long long)g.n * ((pq + 31) / 32) + 3) / 4 * tiles_n, P.cgs) +
+                                        // strided: a gather or scatter pass over the dense copy
+                                        (dense ? 0.0 : 6.0 + 8.0 * g.n * (mode == 0 ? g.c : g.c * g.sr * g.sc) * (double)pq / 5.0e6));
+        if (dense && g.kr == 3 && g.kc == 3 && g.pt == 1 && g.pl == 1 && g.iw == g.ow && g.ih == g.oh && pq % 4 == 0 && pq >= 64 && g.iw <= 61 && P.C >= 32 && P.K >= 32)
+            other = std::min(other, tma_fed_us((long long)g.n * ((pq + BM - 1) / BM) * tiles_n, 9 * P.cgs));
+        if (plan.us > 0.95 * other) return 1;
+    }
+    const int planes = precision == 1 ? 1 : 2;
+    if (mode == 1 && out_zero) {
+        // pixels of dx that no tap reaches (stride larger than the filter) keep the zeros they are owed
+        if ((int)P.ncls < std::min(g.sr, g.ih) * std::min(g.sc, g.iw)) {
+            if (int r = launch_zero_fill(cx, st, out, (size_t)g.n * g.c * g.ih * g.iw)) return r;
+        }
+    }
+    TableArgs T{};
+    T.g = g; T.mode = mode; T.check = 7;
+    T.M_total = 0; T.N_total = P.K; T.K_total = T.K_pad = plan.kblocks * BK;
+    char *tb; bool build;
+    size_t off = 0;
+    auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
+    const size_t o_kA = carve((size_t)T.K_pad * 8), o_rowB = carve((size_t)T.N_total * 4), o_kB = carve((size_t)T.K_pad * 4), o_kC = carve((size_t)T.K_pad * 4);
+    tb = cached_table(dev, table_key(T), off, build);
+    if (!tb) return 1;
+    T.rowA = nullptr; T.outM = nullptr; T.kA = (int2 *)(tb + o_kA); T.rowB = (int *)(tb + o_rowB); T.kB = (int *)(tb + o_kB); T.kC = (int *)(tb + o_kC);
+    if (build) {
+        eb::launch(build_tables_kernel, grid_for((size_t)T.K_pad + T.N_total, 256), 256, 0, st, T);
+        EB_LAUNCH_CHECK("conv_rs(tables)");
+    }
+    PackEntry *entry = nullptr;
+    const size_t image_rows = (size_t)plan.kblocks * P.tiles_n * plan.bn * planes;
+    const float *img = packed_weights(cx, st, dev, table_key(T), plan.bn, precision, w, (size_t)g.k * g.c * g.kr * g.kc * sizeof(float), T.rowB, T.kB,
+                                      plan.kblocks, P.tiles_n, P.K, mode == 1, &entry);
+    const size_t part_bytes = P.splits > 1 ? (size_t)P.ncls * P.tiles_m * P.tiles_n * P.splits * 256 * plan.bn * sizeof(float) : 0;
+    const size_t pack_bytes = img ? 0 : image_rows * 128;
+    if (part_bytes + pack_bytes) {
+        char *ws = (char *)scratch(cx, part_bytes + pack_bytes);
+        if (!ws) return cudaErrorMemoryAllocation;
+        P.part = (float *)(ws + pack_bytes);
+        if (!img) {
+            eb::launch(pack_b_kernel, dim3(plan.kblocks, P.tiles_n), 256, 0, st, w, T.rowB, T.kB, (float *)ws, plan.bn, P.K, P.tiles_n, mode == 1, precision);
+            EB_LAUNCH_CHECK("conv_rs(pack weights)");
+            img = (const float *)ws;
+        }
+    }
+    if (entry && entry->packed == img) {
+        if (!entry->has_map) { if (!encode_rows_map(&entry->map, img, image_rows, plan.bn / 2)) return 1; entry->has_map = true; }
+        P.mapB = entry->map;
+    } else if (!encode_rows_map(&P.mapB, img, image_rows, plan.bn / 2)) return 1;
+    if (int r = status_word(dev, st)) return r;
+    P.status = g_status[dev];
+    P.src = src; P.out = out; P.bias = mode == 0 ? bias : nullptr;
+    P.accumulate = mode == 1 && !out_zero; P.add_zero = mode == 1 && out_zero;
+    const long long total = (long long)P.ncls * P.tiles_m * P.tiles_n * P.splits;
+    const int grid = 2 * (int)(total < EDDLB200_NUM_SMS / 2 ? total : EDDLB200_NUM_SMS / 2);
+    if (precision == 0) return launch_rs_bn<0>(cx, st, P, grid, plan.smem, plan.bn, dev);
+    if (precision == 2) return launch_rs_bn<2>(cx, st, P, grid, plan.smem, plan.bn, dev);
+    return launch_rs_bn<1>(cx, st, P, grid, plan.smem, plan.bn, dev);
 }
 
 // One GEMM launch (tables + main kernel + optional split-K combine).  T carries mode / class fields and the
@@ -1597,7 +1795,9 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     bool atma = g_conv_tma > 0 && (mode == 0 || mode == 1) && g.kr == 1 && g.kc == 1 && g.sr == 1 && g.sc == 1 && g.pt == 0 && g.pl == 0 &&
                 g.ih == g.oh && g.iw == g.ow && pq_ % 4 == 0 && pq_ >= 32 && a_channels >= 32 && o_channels >= 32 &&
                 aligned16(srcA) && aligned16(out) && (long long)g.n * chunks * 32 < 0x7fffffffLL &&
-                (mode == 0 || out_zero || g_conv_tma > 1);
+                (mode == 0 || out_zero || g_conv_tma > 1) &&
+                // a few tiles with a long reduction (one image at 14 x 14): the gather kernel splits the reduction, this one cannot
+                tma_fed_us((long long)(g.n * chunks + 3) / 4 * ((T.N_total + tile_n(T.N_total) - 1) / tile_n(T.N_total)), (a_channels + BK - 1) / BK) < 1.1 * gather_layer_us(g, mode);
     if (atma) {
         P.chunks_per_image = chunks; P.images = g.n;
         if (!encode_plane_map(&P.mapA, srcA, pq_, a_channels, g.n) || !encode_plane_map(&P.mapOut, out, pq_, o_channels, g.n)) atma = false;
@@ -1609,7 +1809,8 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     bool stma = g_conv_tma > 0 && (mode == 0 || mode == 1) && g.kr == 3 && g.kc == 3 && g.sr == 1 && g.sc == 1 && g.pt == 1 && g.pl == 1 &&
                 g.ih == g.oh && g.iw == g.ow && g.iw >= 3 && 2 * g.iw + BM + 5 <= SLAB_PX && pq_ % 4 == 0 && pq_ >= 64 && a_channels >= 32 && o_channels >= 32 &&
                 aligned16(srcA) && aligned16(out) && (long long)g.n * tiles_per_image * BM < 0x7fffffffLL && (mode == 0 || out_zero || g_conv_tma > 1) &&
-                g_conv_tma3;
+                g_conv_tma3 &&
+                tma_fed_us((long long)g.n * tiles_per_image * ((T.N_total + tile_n(T.N_total) - 1) / tile_n(T.N_total)), (a_channels + BK - 1) / BK * 9) < 1.1 * gather_layer_us(g, mode);
     if (stma) {
         P.chunks_per_image = 4 * tiles_per_image; P.images = g.n; P.img_w = g.iw; P.tap_sign = mode == 0 ? 1 : -1;
         if (!encode_plane_map(&P.mapA, srcA, pq_, a_channels, g.n, BK, false, SLAB_PX) || !encode_plane_map(&P.mapOut, out, pq_, o_channels, g.n)) stma = false;
@@ -1635,25 +1836,10 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     // proportion to its length (measured on backward-weight of N=64, 256 channels, 56x56: 2000 k-steps per accumulator
     // gave 3e-5 of the largest gradient).  kMaxChainBlocks K-blocks per split keep every accumulator's chain at about
     // 200 k-steps (a few 1e-6); the partial sums of the splits are added in fp32 with rounding.
-    constexpr int kMaxChainBlocks = 160;
     const int tiles = tiles_m * tiles_n;
     const int sp_min = allow_split ? (kblocks + kMaxChainBlocks - 1) / kMaxChainBlocks : 1;
     int splits = sp_min;
-    if (allow_split && kblocks >= 8) {
-        const double t_kblock = mode == 2 ? 2.5 : 1.0, t_epilogue = 3.0;
-        int max_splits = kblocks / 4 < 128 ? kblocks / 4 : 128;
-        if (max_splits < sp_min) max_splits = sp_min + sp_min / 4;
-        double best = 1e30;
-        for (int sp = sp_min; sp <= max_splits; sp++) {
-            const int kb = (kblocks + sp - 1) / sp;
-            const int sp_eff = (kblocks + kb - 1) / kb;
-            if (sp_eff != sp) continue;
-            const long long rounds = ((long long)tiles * sp + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS;
-            double cost = (double)rounds * (kb * t_kblock + t_epilogue);
-            if (sp > 1) cost += 3.0 + 2.0 * (double)out_total * sizeof(float) * sp / 6.0e6;
-            if (cost < best * 0.97) { best = cost; splits = sp; }      // prefer fewer splits unless the gain is clear
-        }
-    }
+    if (allow_split && kblocks >= 8) splits = pick_splits(tiles, kblocks, mode == 2 ? 2.5 : gather_us(bn), out_total, sp_min).splits;
     const int kbs = (kblocks + splits - 1) / splits;
     splits = (kblocks + kbs - 1) / kbs;
     // one scratch carve-up: tables and split-K partials
@@ -1663,17 +1849,8 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
                  o_kB = carve((size_t)T.K_pad * 4), o_kC = carve((size_t)T.K_pad * 4), o_outM = carve((size_t)T.M_total * 4);
     const size_t table_bytes = off;
     // cached tables live in their own allocation; the scratch arena then holds only partials and packed weights
-    char *tb = nullptr; bool build = true;
-    {
-        TableCache &tc = g_tables[dev];
-        std::lock_guard<std::mutex> lock(tc.mu);
-        const auto key = table_key(T);
-        auto it = tc.entries.find(key);
-        if (it != tc.entries.end()) { tb = it->second; build = false; }
-        else if (tc.bytes + table_bytes <= kTableCacheBudget && cudaMalloc((void **)&tb, table_bytes) == cudaSuccess) {
-            tc.entries.emplace(key, tb); tc.bytes += table_bytes;
-        } else { tb = nullptr; cudaGetLastError(); }
-    }
+    bool build = true;
+    char *tb = cached_table(dev, table_key(T), table_bytes, build);
     if (tb) off = 0;
     const bool tb_cached = tb != nullptr;
     const size_t o_part = carve(splits > 1 ? out_total * splits * sizeof(float) : 0),
@@ -1681,10 +1858,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     char *ws = (char *)scratch(cx, off ? off : 256);
     if (!ws) return cudaErrorMemoryAllocation;
     if (!tb) tb = ws;
-    if (!g_status[dev]) {
-        if (cudaMalloc((void **)&g_status[dev], sizeof(int)) != cudaSuccess) return cudaErrorMemoryAllocation;
-        cudaMemsetAsync(g_status[dev], 0, sizeof(int), st);
-    }
+    if (int r = status_word(dev, st)) return r;
     T.rowA = (int2 *)(tb + o_rowA); T.kA = (int2 *)(tb + o_kA); T.rowB = (int *)(tb + o_rowB); T.kB = (int *)(tb + o_kB); T.outM = (int *)(tb + o_outM); T.kC = (int *)(tb + o_kC);
     if (build) {
         const long long entries = (long long)T.M_total + T.K_pad + T.N_total;
@@ -1915,6 +2089,12 @@ int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const floa
     return run_one(cx, st, dev, T, P, a, b, c, nullptr, precision, (size_t)m * n, true, inc_c == 2);
 }
 
+int conv_tc_rs(DevCtx *cx, cudaStream_t st, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias, int precision, bool out_zero) {
+    if (!fits(g)) return 1;
+    int dev = 0; cudaGetDevice(&dev);
+    return run_rs(cx, st, dev, mode, g, src, w, out, bias, precision, out_zero);
+}
+int conv_tc_set_rs(int level) { g_conv_rs = level; return 0; }
 int conv_tc_set_prefetch(int on) { g_conv_prefetch = on ? 1 : 0; return 0; }
 int conv_tc_set_tma(int level) { g_conv_tma = level < 0 ? 0 : (level > 2 ? 2 : level); return 0; }
 int conv_tc_set_pack_cache(int on) { g_conv_pack_cache = on ? 1 : 0; return 0; }

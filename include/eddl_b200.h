@@ -262,6 +262,9 @@ int eddlb200_reduce_sum2d(int dev, const float *a, float *b, int rows, int cols,
           pixels, at least 32 channels on both sides) are fed by TMA tensor copies of the activations and drained by TMA
           stores, or TMA fp32 adds where the output accumulates; 1 = only where the output is stored; 0 = the gather
           kernel everywhere.  Results are the same bits at every level.
+ *          "conv_pairs" 1 (default) = forward and backward-data of layers with 16 channels or more run on pairs of CTAs that convert
+ *          the activations once for all filter taps, where an estimate says that this is the faster kernel; 2 = wherever it fits;
+ *          0 = never.  The reduction is ordered (channel group, tap, channel): agreement with the other kernels to rounding.
  *          "conv_tma_3x3" 1 (default) = forward and backward-data of 3x3 stride-1 pad-1 layers (planes of a multiple of 4
  *          pixels and at least 64, rows of at most 125 pixels, at least 32 channels on both sides) read raw slabs of the
  *          activations delivered by TMA, one per tile and 32-channel group for all nine taps; the reduction is then
