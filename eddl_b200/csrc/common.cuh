@@ -79,15 +79,29 @@ int launch_zero_fill(DevCtx *c, cudaStream_t st, float *p, size_t n);    // defi
 // activation that follows LAdd in a residual block -- one kernel writes both the sum and its ReLU (16 bytes per element instead
 // of 12 + 8); again any other entry point first runs what is on record.  LAdd::backward adds its delta into the (zero) deltas of
 // both parents: the second such copy FROM THE SAME SOURCE joins the record (kind 3) and one kernel reads the source once.
+// The ReLU backward pass into a delta known to hold zeros is recorded as well (kind 4): the BatchNorm backward pass that follows
+// it in every conv-BN-ReLU chain takes it over and masks the delta as it reads it (bn.cu).  When copies of that delta into the
+// zero deltas of both parents of an LAdd come next, they join the record (kind 5) and one kernel writes all three.
 struct PendCopy {
     bool active = false; int kind = 1;                   // 1: dst = sa*src + sb*0     2: dst = s2*src2 + t2*(sa*src + sb*0)
                                                          // 3: dst = dst2 = sa*src + sb*0   (LAdd::backward: the delta into both parents)
-    float *dst = nullptr, *dst2 = nullptr; const float *src = nullptr, *src2 = nullptr;
+                                                         // 4: dst = src2 > 0 ? src : 0     (ReLU backward)
+                                                         // 5: the same; dst2 (and dst3) = sa*dst + sb*0
+    float *dst = nullptr, *dst2 = nullptr, *dst3 = nullptr; const float *src = nullptr, *src2 = nullptr;
     float sa = 0.f, sb = 0.f, s2 = 0.f, t2 = 0.f; size_t n = 0;
 };
 bool pend_copy_active(DevCtx *c);
 PendCopy &pend_copy(DevCtx *c);
 int pend_copy_flush(DevCtx *c, cudaStream_t st);                         // defined with the elementwise kernels
+
+// What a BatchNorm output was computed from, so that a ReLU backward pass that tests it can be folded into the BatchNorm backward
+// pass without reading it: y = opa * g + b has the same bits when it is computed again.  Valid while none of the four
+// tensors has been written (write observers).
+struct BnSource { const float *opa = nullptr, *g = nullptr, *b = nullptr; size_t n = 0; unsigned long long vy = 0, vopa = 0, vg = 0, vb = 0; };
+void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z);
+// b of y = opa * g + b when y is still that, else nullptr
+const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n);
+bool lz_enabled(DevCtx *c);
 
 }  // namespace eb
 

@@ -92,6 +92,30 @@ __global__ void __launch_bounds__(kBlock) map1_twice_kernel(const float *a, floa
     for (size_t j = 4 * n4 + i; j < n; j += stride) { const float v = f(a[j]); b[j] = v; c[j] = v; }
 }
 
+// m = i > 0 ? 0 + d : 0; b = c = f(m): a recorded ReLU backward pass together with the copies of its result into one or two other
+// deltas (c may be null).  n4 = 0 runs everything in the scalar loop.
+template <typename F>
+__global__ void __launch_bounds__(kBlock) relu_bwd_copies_kernel(const float *d, const float *i, float *m, float *b, float *c, size_t n4, size_t n, F f) {
+    EB_GRID_WAIT();
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t j = first; j < n4; j += stride) {
+        float4 v = *reinterpret_cast<const float4 *>(d + 4 * j);
+        const float4 x = *reinterpret_cast<const float4 *>(i + 4 * j);
+        v.x = x.x > 0.f ? __fadd_rn(0.f, v.x) : 0.f; v.y = x.y > 0.f ? __fadd_rn(0.f, v.y) : 0.f;
+        v.z = x.z > 0.f ? __fadd_rn(0.f, v.z) : 0.f; v.w = x.w > 0.f ? __fadd_rn(0.f, v.w) : 0.f;
+        *reinterpret_cast<float4 *>(m + 4 * j) = v;
+        v.x = f(v.x); v.y = f(v.y); v.z = f(v.z); v.w = f(v.w);
+        *reinterpret_cast<float4 *>(b + 4 * j) = v;
+        if (c) *reinterpret_cast<float4 *>(c + 4 * j) = v;
+    }
+    for (size_t j = 4 * n4 + first; j < n; j += stride) {
+        const float v = i[j] > 0.f ? __fadd_rn(0.f, d[j]) : 0.f, w = f(v);
+        m[j] = v; b[j] = w;
+        if (c) c[j] = w;
+    }
+}
+
 template <typename F>
 int launch1(DevCtx *cx, cudaStream_t st, const float *a, float *b, size_t n, F f, const char *what, double bytes_per_element = 8.0) {
     if (n == 0) return 0;
@@ -252,6 +276,17 @@ int pend_copy_flush(DevCtx *cx, cudaStream_t st) {
         EB_LAUNCH_CHECK("gpu_add (two destinations)");
         return 0;
     }
+    if (p.kind == 4) return launch3(cx, st, p.src, p.src2, p.dst, p.n, ReluBwdZeroF{}, "gpu_d_relu", 12.0);
+    if (p.kind == 5) {
+        const size_t n = p.n;
+        EB_READS(p.src, n * sizeof(float)); EB_READS(p.src2, n * sizeof(float)); EB_WRITES(p.dst, n * sizeof(float)); EB_WRITES(p.dst2, n * sizeof(float));
+        if (p.dst3) EB_WRITES(p.dst3, n * sizeof(float));
+        ProfScope prof(cx, PROF_ELEMENTWISE, (p.dst3 ? 20.0 : 16.0) * n);
+        const size_t n4 = (aligned16(p.src) && aligned16(p.src2) && aligned16(p.dst) && aligned16(p.dst2) && (!p.dst3 || aligned16(p.dst3))) ? n / 4 : 0;
+        eb::launch(relu_bwd_copies_kernel<AxpbZeroF>, grid_for(n4 ? n4 : n, kBlock), kBlock, 0, st, p.src, p.src2, p.dst, p.dst2, p.dst3, n4, n, AxpbZeroF{p.sa, p.sb});
+        EB_LAUNCH_CHECK("gpu_d_relu + gpu_add");
+        return 0;
+    }
     return launch1(cx, st, p.src, p.dst, p.n, AxpbZeroF{p.sa, p.sb}, "gpu_add", 8.0);
 }
 // writes n zeros at p; used when a deferred zero fill has to be materialised
@@ -345,6 +380,16 @@ int eddlb200_axpby(int dev, float sca, const float *a, float scb, const float *b
             if (lz_take(cx, st, c, n * sizeof(float), &status)) { p.kind = 3; p.dst2 = c; return 0; }
             if (status) return status;
         }
+        if ((p.kind == 4 || (p.kind == 5 && !p.dst3)) && !inc_c && c && c == b && a == p.dst && n == p.n && c != p.dst && c != p.dst2 && c != p.src && c != p.src2 && lz_any(cx) &&
+            (p.kind == 4 || (sca == p.sa && scb == p.sb))) {
+            // the delta of a recorded ReLU backward pass copied into another zero delta: it joins the record
+            int status = 0;
+            if (lz_take(cx, st, c, n * sizeof(float), &status)) {
+                if (p.kind == 4) { p.kind = 5; p.dst2 = c; p.dst3 = nullptr; p.sa = sca; p.sb = scb; } else p.dst3 = c;
+                return 0;
+            }
+            if (status) return status;
+        }
         if (int r = pend_copy_flush(cx, st)) return r;
     }
     if (inc_c && c && c != a && c != b && lz_any(cx)) {
@@ -360,7 +405,8 @@ int eddlb200_axpby(int dev, float sca, const float *a, float scb, const float *b
             if (c == b) {
                 // record instead of run: the next call is usually the second term of the same sum
                 PendCopy &p = pend_copy(cx);
-                p.active = true; p.kind = 1; p.dst = c; p.src = a; p.src2 = nullptr; p.sa = sca; p.sb = scb; p.n = n;
+                p = PendCopy{};
+                p.active = true; p.kind = 1; p.dst = c; p.src = a; p.sa = sca; p.sb = scb; p.n = n;
                 return 0;
             }
             return launch1(cx, st, b, c, n, ZeroAxpbF{sca, scb}, "gpu_add", 8.0);
@@ -395,7 +441,14 @@ int eddlb200_relu_bwd(int dev, const float *d, const float *i, float *pd, size_t
     EB_CTX(dev);
     if (pd && pd != d && pd != i && lz_any(cx)) {
         int status = 0;
-        if (lz_take(cx, st, pd, n * sizeof(float), &status)) return launch3(cx, st, d, i, pd, n, ReluBwdZeroF{}, "gpu_d_relu", 12.0);
+        if (lz_take(cx, st, pd, n * sizeof(float), &status)) {
+            if (!d || !i) return set_error(EDDLB200_EINVAL, "gpu_d_relu: null pointer");
+            // recorded for one call: the BatchNorm backward pass or the copies that usually follow take it over
+            PendCopy &p = pend_copy(cx);
+            p = PendCopy{};
+            p.active = true; p.kind = 4; p.dst = pd; p.src = d; p.src2 = i; p.n = n;
+            return 0;
+        }
         if (status) return status;
     }
     return launch3(cx, st, d, i, pd, n, ReluBwdF{}, "gpu_d_relu");

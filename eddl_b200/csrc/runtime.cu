@@ -43,6 +43,7 @@ struct DevCtx {
     bool lz_on = false;
     std::map<uintptr_t, size_t> lz;
     PendCopy pend;
+    std::unordered_map<const float *, BnSource> bn_sources;
     // write observers: start address -> (bytes, version)
     struct Watch { size_t bytes; unsigned long long version; };
     std::map<uintptr_t, Watch> watch;
@@ -263,6 +264,24 @@ void watch_forget(DevCtx *c, const void *p, size_t bytes) {
     for (uintptr_t k : gone) c->watch.erase(k);
 }
 
+void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z) {
+    if (c->bn_sources.size() > 4096) c->bn_sources.clear();            // nets that are gone leave entries behind
+    BnSource s;
+    s.opa = opa; s.g = g; s.b = b; s.n = n;
+    watch_add(c, y, n * sizeof(float)); watch_add(c, opa, n * sizeof(float)); watch_add(c, g, z * sizeof(float)); watch_add(c, b, z * sizeof(float));
+    // overlapping ranges evict each other: read the versions once all four are registered (0 = not observed)
+    s.vy = watch_version(c, y); s.vopa = watch_version(c, opa); s.vg = watch_version(c, g); s.vb = watch_version(c, b);
+    c->bn_sources[y] = s;
+}
+const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n) {
+    auto it = c->bn_sources.find(y);
+    if (it == c->bn_sources.end()) return nullptr;
+    const BnSource &s = it->second;
+    const bool same = s.opa == opa && s.g == g && s.n == n && s.vy && s.vopa && s.vg && s.vb && watch_version(c, y) == s.vy && watch_version(c, opa) == s.vopa &&
+                      watch_version(c, g) == s.vg && watch_version(c, s.b) == s.vb;
+    return same ? s.b : nullptr;
+}
+
 // ---- deferred zero fills ------------------------------------------------------------------------------
 constexpr size_t kLazyZeroMinBytes = size_t(256) << 10;      // smaller fills are cheaper to run (batched) than to track
 
@@ -270,6 +289,7 @@ constexpr size_t kLazyZeroMinBytes = size_t(256) << 10;      // smaller fills ar
 static struct LzStats { unsigned long long deferred = 0, taken = 0, dropped = 0, written = 0; double written_bytes = 0, deferred_bytes = 0;
     ~LzStats() { if (getenv("EDDL_B200_LZ_STATS")) fprintf(stderr, "[lazy_zero] deferred %llu (%.1f MB) taken %llu dropped %llu written %llu (%.1f MB)\n", deferred, deferred_bytes / 1e6, taken, dropped, written, written_bytes / 1e6); } } g_lzs;
 bool lz_any(DevCtx *c) { return !c->lz.empty(); }
+bool lz_enabled(DevCtx *c) { return c->lz_on; }
 bool pend_copy_active(DevCtx *c) { return c->pend.active; }
 PendCopy &pend_copy(DevCtx *c) { return c->pend; }
 
@@ -615,7 +635,8 @@ int eddlb200_profile_reset(int dev) {
 }
 
 int eddlb200_launch_count(int dev, unsigned long long *n) {
-    EB_CTX_KEEP_PENDING(dev);       // a pure counter read: it does not touch device memory
+    EB_CTX_KEEP_PENDING(dev);       // a counter read: it does not touch device memory; a recorded ReLU backward pass is a call of the past and counts
+    if (cx->pend.active && cx->pend.kind >= 4) { if (int r = pend_copy_flush(cx, st)) return r; }
     if (!n) return set_error(EDDLB200_EINVAL, "launch_count: null");
     *n = cx->launches;
     return 0;
