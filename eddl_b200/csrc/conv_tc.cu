@@ -49,6 +49,7 @@
 #include "conv_common.cuh"
 #include "tc_ptx.cuh"
 #include "conv_rs.cuh"
+#include "conv_wg.cuh"
 
 namespace {
 
@@ -61,10 +62,6 @@ constexpr int NTHREADS = NPROD + 32 + NEPI + 32;     // + warp 13: L2 prefetch o
 // output-heavy layers are bound by the epilogue's chain of tensor-memory reads, and two warps per lane quarter halve it
 constexpr int NTHREADS_ATMA = NTHREADS + NEPI;
 constexpr int threads_of(int tma) { return (tma == 1 || tma == 3) ? NTHREADS_ATMA : NTHREADS; }
-// backward-weight of 3x3 stride-1 pad-1 layers fed from raw slabs (TMA = 4): a tile's 128 rows are the nine taps of 14 channels
-// (126 rows, the last two stay zero) and a K-block is 32 pixels of one image; one slab of [16 channels][152 pixels] -- the 32
-// pixels plus a halo of W + 1 either side, its start rounded down to 16 bytes -- serves all 126 rows (W <= 57)
-constexpr int WS_CH = 14, WS_ROWS = 9 * WS_CH, WS_SLAB_PX = 152, WS_SLAB_CH = 16;
 constexpr int SLAB_PX = 256;        // pixels per channel of a raw slab (3x3 TMA-fed kernels): 128 rows + a halo of W + 1 either side + alignment
 constexpr int PF_AHEAD = 8;         // K-blocks the prefetch warp may run ahead of the producers
 constexpr int INVALID_Y = -20000;
@@ -1521,9 +1518,9 @@ int launch_rs_bn(DevCtx *cx, cudaStream_t st, const RsParams &P, int grid, int s
 // ---- which kernel: estimates in microseconds, calibrated on the layers of the nets at batch 1 to 128 ----
 constexpr int kMaxChainBlocks = 160;       // K-blocks per split: see the accumulator drift in run_one
 struct SplitChoice { int splits; double us; };
-// Split the reduction of `tiles` output tiles over the SMs: the makespan of `tiles * splits` work items dealt round-robin is
+// Split the reduction of `tiles` output tiles over the SMs (units: SMs or pairs of them): the makespan of `tiles * splits` work items dealt round-robin is
 // ceil(items / SMs) rounds of (K-blocks per split + one epilogue); splitting also costs a write and a read of every partial output.
-SplitChoice pick_splits(long long tiles, int kblocks, double t_kblock, size_t out_total, int sp_min) {
+SplitChoice pick_splits(long long tiles, int kblocks, double t_kblock, size_t out_total, int sp_min, int units = EDDLB200_NUM_SMS) {
     const double t_epilogue = 3.0;
     int max_splits = kblocks / 4 < 128 ? kblocks / 4 : 128;
     if (max_splits < sp_min) max_splits = sp_min + sp_min / 4;
@@ -1531,12 +1528,12 @@ SplitChoice pick_splits(long long tiles, int kblocks, double t_kblock, size_t ou
     for (int sp = sp_min; sp <= max_splits; sp++) {
         const int kb = (kblocks + sp - 1) / sp;
         if ((kblocks + kb - 1) / kb != sp) continue;
-        const long long rounds = (tiles * sp + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS;
+        const long long rounds = (tiles * sp + units - 1) / units;
         double cost = (double)rounds * (kb * t_kblock + t_epilogue);
         if (sp > 1) cost += 3.0 + 2.0 * (double)out_total * sizeof(float) * sp / 6.0e6;
         if (cost < best.us * 0.97) best = SplitChoice{sp, cost};          // prefer fewer splits unless the gain is clear
     }
-    if (best.us >= 1e30) best.us = (double)((tiles * sp_min + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS) * ((double)kblocks / sp_min * t_kblock + t_epilogue);
+    if (best.us >= 1e30) best.us = (double)((tiles * sp_min + units - 1) / units) * ((double)kblocks / sp_min * t_kblock + t_epilogue);
     return best;
 }
 inline int tile_n(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : 128); }
@@ -1737,6 +1734,87 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
     return launch_rs_bn<1>(cx, st, P, grid, plan.smem, plan.bn, dev);
 }
 
+template <int BN_, bool SPLIT3, bool SLAB>
+int launch_wg(DevCtx *cx, cudaStream_t st, const WgParams &P, int grid, int dev) {
+    constexpr int SMEM = WgLayout<BN_, SPLIT3, SLAB>::SMEM_BYTES;
+    static bool configured_dev[EDDLB200_MAX_DEVICES] = {};
+    if (!configured_dev[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(conv_wg_kernel<BN_, SPLIT3, SLAB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return cuda_status(e, "conv_wg(smem attribute)");
+        configured_dev[dev] = true;
+    }
+    eb::launch(conv_wg_kernel<BN_, SPLIT3, SLAB>, grid, WG_THREADS, SMEM, st, P);
+    EB_LAUNCH_CHECK("conv_wg");
+    return 0;
+}
+template <bool SPLIT3, bool SLAB>
+int launch_wg_bn(DevCtx *cx, cudaStream_t st, const WgParams &P, int grid, int bn, int dev) {
+    if (bn == 32) return launch_wg<32, SPLIT3, SLAB>(cx, st, P, grid, dev);
+    if (bn == 64) return launch_wg<64, SPLIT3, SLAB>(cx, st, P, grid, dev);
+    return launch_wg<128, SPLIT3, SLAB>(cx, st, P, grid, dev);
+}
+
+// Sum of the split-K partials, stored or added.
+int combine_splits(DevCtx *cx, cudaStream_t st, const float *part, float *out, size_t out_total, int splits, bool store, const float *bias, int plane, int nbias) {
+    if (!store) return splitk_reduce_accumulate(cx, st, part, out, out_total, splits);
+    // `out` holds nothing to add to: store the sum of the partials (0 + p0 + p1 + ...)
+    eb::launch(splitk_store_kernel, grid_for(out_total, 256), 256, 0, st, part, out, out_total, splits, bias, plane, nbias);
+    EB_LAUNCH_CHECK("conv_tc(split-K store)");
+    return 0;
+}
+
+// Backward-weight on CTA pairs (conv_wg.cuh) of a layer that the TMA-fed kernels take (slab: 3x3 "same", otherwise 1x1 dense); 1 = the
+// kernel on single CTAs is the faster one.  A pair has twice the rows of a CTA, so a layer with few rows leaves half of it empty,
+// and half as many units to fill: both estimates are made with the splits that each would choose.
+int run_wg(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool slab, bool gw_zero) {
+    if (!g_conv_rs) return 1;
+    const int pq = g.oh * g.ow, chunks = (pq + 31) / 32, kblocks = g.n * chunks, sp_min = (kblocks + kMaxChainBlocks - 1) / kMaxChainBlocks;
+    const size_t out_total = (size_t)g.k * g.c * g.kr * g.kc;
+    auto kblock_us = [&](int bn, bool pairs) {
+        // 3xTF32, microseconds per K-block of a CTA, from ResNet-50's layers at batch 64
+        const double f = precision == 1 ? 0.6 : 1.0;
+        if (slab) return f * (pairs ? (bn == 128 ? 0.94 : 0.72) : (bn == 128 ? 1.05 : 0.80));
+        return f * (pairs ? (bn == 128 ? 0.70 : 0.55) : (bn == 128 ? 0.90 : 0.75));
+    };
+    // rows x columns: (channel, tap) x filter; 1x1 layers may also take filter x channel
+    struct Plan { int tiles_m, bn, tiles_n; bool swap; SplitChoice c; };
+    auto plan = [&](bool swap, bool pairs) {
+        Plan p;
+        const int rows = slab ? (g.c + WS_CH - 1) / WS_CH * BM : swap ? g.k : g.c, cols = swap ? g.c : g.k, per = pairs ? 2 * BM : BM;
+        p.swap = swap; p.tiles_m = (rows + per - 1) / per; p.bn = tile_n(cols); p.tiles_n = (cols + p.bn - 1) / p.bn;
+        p.c = pick_splits((long long)p.tiles_m * p.tiles_n, kblocks, kblock_us(p.bn, pairs), out_total, sp_min, pairs ? EDDLB200_NUM_SMS / 2 : EDDLB200_NUM_SMS);
+        return p;
+    };
+    Plan p = plan(false, true);
+    if (!slab) { const Plan q = plan(true, true); if (q.c.us < 0.98 * p.c.us) p = q; }
+    if (g_conv_rs < 2 && p.c.us > 0.97 * plan(false, false).c.us) return 1;
+    WgParams P{};
+    const float *a = p.swap ? dy : x, *b = p.swap ? x : dy;
+    const int ca = p.swap ? g.k : g.c, cb = p.swap ? g.c : g.k;
+    const bool maps = slab ? encode_plane_map(&P.mapA, a, pq, ca, g.n, WS_SLAB_CH, false, WS_SLAB_PX) : encode_plane_map(&P.mapA, a, pq, ca, g.n, BM, true);
+    if (!maps || !encode_plane_map(&P.mapB, b, pq, cb, g.n, p.bn / 2, true)) return 1;
+    const int kbs = (kblocks + p.c.splits - 1) / p.c.splits, splits = (kblocks + kbs - 1) / kbs;
+    if (int r = status_word(dev, st)) return r;
+    float *part = splits > 1 ? (float *)scratch(cx, out_total * splits * sizeof(float)) : nullptr;
+    if (splits > 1 && !part) return cudaErrorMemoryAllocation;
+    P.status = g_status[dev];
+    P.out = splits > 1 ? part : gw; P.split_stride = splits > 1 ? (long long)out_total : 0; P.accumulate = splits == 1 && !gw_zero;
+    const int row_elems = g.c * g.kr * g.kc;
+    P.m_stride = p.swap ? row_elems : 1; P.n_stride = p.swap ? 1 : row_elems;
+    P.M_total = slab ? row_elems : ca; P.N_total = cb;
+    P.tiles_m = p.tiles_m; P.tiles_n = p.tiles_n; P.splits = splits; P.kblocks = kblocks; P.kblocks_per_split = kbs;
+    P.chunks_per_image = chunks; P.img_w = g.iw; P.plane_px = pq; P.raw_hi = g_conv_wtma > 1;
+    P.nmain = kbs * (BK / 8) > 64 ? NMAIN : 1;                            // as in run_one
+    const long long total = (long long)p.tiles_m * p.tiles_n * splits;
+    const int grid = 2 * (int)(total < EDDLB200_NUM_SMS / 2 ? total : EDDLB200_NUM_SMS / 2);
+    int r;
+    // backward-weight has no bf16 variant: precision 2 runs it as precision 0
+    if (slab) r = precision != 1 ? launch_wg_bn<true, true>(cx, st, P, grid, p.bn, dev) : launch_wg_bn<false, true>(cx, st, P, grid, p.bn, dev);
+    else r = precision != 1 ? launch_wg_bn<true, false>(cx, st, P, grid, p.bn, dev) : launch_wg_bn<false, false>(cx, st, P, grid, p.bn, dev);
+    if (r || splits == 1) return r;
+    return combine_splits(cx, st, part, gw, out_total, splits, gw_zero, nullptr, 1, 1);
+}
+
 // One GEMM launch (tables + main kernel + optional split-K combine).  T carries mode / class fields and the
 // problem extents; out_total is the element count of the output tensor (the unit of a split-K partial).
 int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const float *srcA, const float *srcB, float *out,
@@ -1767,6 +1845,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     bool wtma = planes_dense && g_conv_wtma > 0 && g.oh * g.ow >= 32 && g.c >= 32 && g.k >= 32;
     int w_bn = 0;
     if (wtma) {
+        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, false, out_zero); r != 1) return r;
         w_bn = T.N_total <= 32 ? 32 : (T.N_total <= 64 ? 64 : 128);
         P.chunks_per_image = w_chunks; P.images = g.n; P.raw_hi = g_conv_wtma > 1;
         if (!encode_plane_map(&P.mapA, srcA, g.oh * g.ow, g.c, g.n, BM, true) || !encode_plane_map(&P.mapOut, srcB, g.oh * g.ow, g.k, g.n, w_bn, true)) wtma = false;
@@ -1779,6 +1858,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
                  g.ih == g.oh && g.iw == g.ow && g.iw >= 3 && 2 * (g.iw + 1) + BK + 3 <= WS_SLAB_PX && (g.oh * g.ow) % 4 == 0 && g.oh * g.ow >= 32 &&
                  g.c >= WS_CH && g.k >= 32 && aligned16(srcA) && aligned16(srcB);
     if (wslab) {
+        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, true, out_zero); r != 1) return r;
         const int ws_bn = T.N_total <= 32 ? 32 : (T.N_total <= 64 ? 64 : 128);
         P.chunks_per_image = w_chunks; P.images = g.n; P.raw_hi = g_conv_wtma > 1; P.img_w = g.iw; P.plane_px = g.oh * g.ow;
         if (!encode_plane_map(&P.mapA, srcA, g.oh * g.ow, g.c, g.n, WS_SLAB_CH, false, WS_SLAB_PX) ||
@@ -1909,15 +1989,9 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     else if (precision == 2) r = launch_bn<2, false>(cx, st, P, grid, bn, dev);
     else r = launch_bn<1, false>(cx, st, P, grid, bn, dev);
     if (r) return r;
-    if (splits > 1) {
-        if (mode == 0 || out_zero || (mode == 4 && T.ca != 1)) {
-            // `out` holds nothing to add to: store the sum of the partials (0 + p0 + p1 + ...)
-            eb::launch(splitk_store_kernel, grid_for(out_total, 256), 256, 0, st, (const float *)(ws + o_part), out, out_total, splits, mode == 0 ? bias : nullptr, g.oh * g.ow, g.k);
-            EB_LAUNCH_CHECK("conv_tc(split-K store)");
-            return 0;
-        }
-        return splitk_reduce_accumulate(cx, st, (const float *)(ws + o_part), out, out_total, splits);
-    }
+    if (splits > 1)
+        return combine_splits(cx, st, (const float *)(ws + o_part), out, out_total, splits, mode == 0 || out_zero || (mode == 4 && T.ca != 1), mode == 0 ? bias : nullptr,
+                              g.oh * g.ow, g.k);
     return 0;
 }
 
