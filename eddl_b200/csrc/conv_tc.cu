@@ -197,6 +197,8 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * STAGES + 4 + XBARS);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     volatile int *progress = abort_flag + 1;              // last K-block (CTA sequence number) producer group 0 has stored
+    // ATMA: one word per producer warp follows (release_raw)
+    static_assert(!ATMA || (2 * STAGES + 4 + 2 * RAWS) * 8 + 12 + 8 * 4 <= 256, "barrier words");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kb_total = P.K_pad / BK;
@@ -435,6 +437,20 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
             // STMA state of this thread's row: position of the row inside the slab for the centre tap, and whether the row's
             // pixel sits on the left / right edge of the image (its horizontal neighbours then lie in another image row)
             int slab_pos = 0; bool edge_l = false, edge_r = false;
+            // Hands a landing slot back to TMA once av[] has been read out of it.  The arrival alone does not order these loads before
+            // the copy that refills the slot: they are generic-proxy reads and the copy writes through the async proxy, and a load
+            // that has been issued but not yet served (shared memory is the bottleneck here, so its queue is long) would return
+            // data of a later K-block.  So the values are USED first -- a store of their OR cannot issue before the last of them is in
+            // its register -- and every lane fences the proxies before lane 0 arrives for the warp.
+            auto release_raw = [&](uint32_t bar) {
+                uint32_t used = 0;
+#pragma unroll
+                for (int i = 0; i < BK; i++) used |= __float_as_uint(av[i]);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(smem_u32((const void *)(progress + 1 + warp))), "r"(used) : "memory");
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar);
+            };
             auto load_row = [&](int t, int kb0, int it, int gseq) -> bool {
                 if constexpr (STMA) {
                     // K-blocks come as (32-channel group, tap): the nine taps of a group read the SAME raw slab
@@ -460,10 +476,7 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
                     const float *raw = (const float *)(raw_base + rs * (2 * L::RAW_BYTES)) + slab_pos + dr * P.img_w + dc;
 #pragma unroll
                     for (int i = 0; i < BK; i++) av[i] = masked ? 0.f : raw[i * SLAB_PX];
-                    if (gseq + 2 > 9 * ss + 8) {            // this group's last K-block of the slab
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_raw_empty + 8 * rs);
-                    }
+                    if (gseq + 2 > 9 * ss + 8) release_raw(bar_raw_empty + 8 * rs);      // this group's last K-block of the slab
                     return true;
                 } else if constexpr (ATMA) {
                     // this thread's row of K-block number gseq of the CTA's sequence: 32 values, one per channel, out of the raw
@@ -473,8 +486,7 @@ __global__ void __launch_bounds__(threads_of(TMA), 1) igemm_tc_kernel(const __gr
                     const float *raw = (const float *)(raw_base + rs * L::RAW_BYTES) + (warp & 3) * (BK * 32) + lane;
 #pragma unroll
                     for (int i = 0; i < BK; i++) av[i] = raw[i * 32];
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_raw_empty + 8 * rs);       // this warp has read its chunk
+                    release_raw(bar_raw_empty + 8 * rs);                      // this warp has read its chunk
                     return true;
                 }
                 const int mn = t % tiles_mn;
