@@ -102,6 +102,12 @@ template <int MASK> __device__ __forceinline__ float4 masked4(float4 d, float4 o
     return make_float4(masked<MASK>(d.x, o.x, i.x, g, b), masked<MASK>(d.y, o.y, i.y, g, b), masked<MASK>(d.z, o.z, i.z, g, b), masked<MASK>(d.w, o.w, i.w, g, b));
 }
 
+// Terms of sum(d * o), with the roundings spelled out: the compiler's own choice of fused multiply-adds differs between the variants
+// with and without a mask, and the folded backward pass has to give the bits of the separate calls.
+__device__ __forceinline__ float dot4(float4 d, float4 o) {
+    return __fadd_rn(__fmaf_rn(d.x, o.x, __fmul_rn(d.y, o.y)), __fmaf_rn(d.z, o.z, __fmul_rn(d.w, o.w)));
+}
+
 // ---- reductions -----------------------------------------------------------------
 // MODE 0: (sum x, sum x*x)      MODE 1: (sum d*o, sum d)
 template <int MODE, bool VEC, int MASK = 0>
@@ -126,7 +132,7 @@ __global__ void __launch_bounds__(kBlock) bn_stats_kernel(const float *__restric
             } else {
                 const float4 w = ldg4(o + off);
                 if (MASK) v = masked4<MASK>(v, w, MASK == 1 ? ldg4(act + off) : w, gj, bj);
-                a0 += (v.x * w.x + v.y * w.y) + (v.z * w.z + v.w * w.w);
+                a0 = __fadd_rn(a0, dot4(v, w));
                 a1 += (v.x + v.y) + (v.z + v.w);
             }
         }
@@ -139,7 +145,7 @@ __global__ void __launch_bounds__(kBlock) bn_stats_kernel(const float *__restric
             else {
                 const float w = o[off];
                 if (MASK) v = masked<MASK>(v, w, MASK == 1 ? act[off] : w, gj, bj);
-                a0 += v * w; a1 += v;
+                a0 = __fmaf_rn(v, w, a0); a1 += v;
             }
         }
     }
@@ -469,13 +475,13 @@ __global__ void __launch_bounds__(kOneBlock) bn_bwd_one_kernel(float *delta, con
                 float4 v = *reinterpret_cast<const float4 *>(bd + t);
                 const float4 w = *reinterpret_cast<const float4 *>(bo + t);
                 if (MASK) { v = masked4<MASK>(v, w, MASK == 1 ? *reinterpret_cast<const float4 *>(ba + t) : w, gj, bj); *reinterpret_cast<float4 *>(bd + t) = v; }
-                a0 += (v.x * w.x + v.y * w.y) + (v.z * w.z + v.w * w.w);
+                a0 = __fadd_rn(a0, dot4(v, w));
                 a1 += (v.x + v.y) + (v.z + v.w);
             } else {
                 float v = bd[t];
                 const float w = bo[t];
                 if (MASK) { v = masked<MASK>(v, w, MASK == 1 ? ba[t] : w, gj, bj); bd[t] = v; }
-                a0 += v * w; a1 += v;
+                a0 = __fmaf_rn(v, w, a0); a1 += v;
             }
         }
         const float2 sum = cluster_totals(a0, a1, c.csize, sm, slot + (k & 1), total + (k & 1));

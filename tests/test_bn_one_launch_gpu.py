@@ -1,5 +1,7 @@
 """GPU parity of BatchNorm where a channel is kept in the shared memory of a cluster, at the edges of its shares and block sizes, against
 the restatement of the reference's arithmetic; the quotients by sigma against IEEE division; the ReLU backward pass folded in."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -8,6 +10,12 @@ from oracle import eddl_oracle as orc
 pytestmark = pytest.mark.gpu
 F = np.float32
 SHAPES = [(1, 1, 1, 1), (2, 3, 1, 2), (5, 7, 7, 7), (3, 33, 2, 2), (4, 5, 9, 13), (64, 2, 28, 28), (3, 300, 10, 10), (16, 3, 64, 64), (2, 4, 113, 115), (129, 2, 100, 36), (40, 2, 256, 256)]
+
+
+def launches(L):
+    n = ctypes.c_ulonglong()
+    L.call("launch_count", 0, ctypes.byref(n))
+    return n.value
 
 
 def _forward(L, x, g, b, relu=True):
@@ -72,14 +80,17 @@ def test_relu_backward_folded_in(lib, shape, own):
             dd, pd, gg, gb, m1, m2 = L.empty(shape), L.empty(shape), L.zeros((z,)), L.zeros((z,)), L.empty((z,)), L.empty((z,))
             for a in (dd, pd):
                 L.call("fill", 0, a, E, 5.0); L.call("fill", 0, a, E, 0.0)
-            L.call("relu_bwd", 0, L.to_device(d), act, dd, E)
+            src, before = L.to_device(d), launches(L)        # kept alive: releasing it would run the record
+            L.call("relu_bwd", 0, src, act, dd, E)
             L.call("bn_bwd", 0, n, z, h * w, dd, opa, pd, gg, gb, dg, va, m1, m2)
-            return [t.numpy() for t in (dd, pd, gg, gb, m1, m2)]
+            return launches(L) - before, [t.numpy() for t in (dd, pd, gg, gb, m1, m2)]
         finally:
             L.call("set_option", b"lazy_zero", 0)
     for overwrite in (False, True):
-        for got, want in zip(run(1, overwrite), run(0, overwrite)):
-            np.testing.assert_array_equal(got, want)
+        (folded, got), (separate, want) = run(1, overwrite), run(0, overwrite)
+        assert folded == separate - 1                       # relu_bwd was taken over
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
 
 
 def test_relu_backward_with_copies(lib):
