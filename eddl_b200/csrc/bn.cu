@@ -657,7 +657,7 @@ int eddlb200_bn_fwd(int dev, int b, int z, int rc, const float *input, float *ou
     const Stride w = stride_of(z, rc, vec ? kBlock * 4 : kBlock);
     dim3 grid(z, S);
     float2 *partial = nullptr;
-    if (trmode && affine_g && opa && lz_enabled(cx)) bn_source_set(cx, output, opa, affine_g, affine_b, (size_t)b * z * rc, z);
+    if (trmode && affine_g && opa && lz_enabled(cx)) bn_source_set(cx, output, opa, affine_g, affine_b, (size_t)b * z * rc, z, rc);
     if (trmode) {
         const int r = fwd_one_launch(dev, st, b, z, rc, vec, input, output, opa, global_mean, global_variance, affine_g, affine_b, mean, variance, epsilon, momentum, relu_out);
         if (r == 0) count_launch(cx);
@@ -689,7 +689,7 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
             // the ReLU backward pass that makes this delta is still on record: it is folded in
             p.active = false;
             src = p.src; act = p.src2;
-            beta = bn_g ? bn_source_beta(cx, act, opa, bn_g, elements) : nullptr;
+            beta = bn_g ? bn_source_beta(cx, act, opa, bn_g, elements, z, rc) : nullptr;
             mask = beta ? 2 : 1;
         } else if (int r = pend_copy_flush(cx, st)) return r;
     }

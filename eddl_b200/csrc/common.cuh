@@ -96,11 +96,11 @@ int pend_copy_flush(DevCtx *c, cudaStream_t st);                         // defi
 
 // What a BatchNorm output was computed from, so that a ReLU backward pass that tests it can be folded into the BatchNorm backward
 // pass without reading it: y = opa * g + b has the same bits when it is computed again.  Valid while none of the four
-// tensors has been written (write observers).
-struct BnSource { const float *opa = nullptr, *g = nullptr, *b = nullptr; size_t n = 0; unsigned long long vy = 0, vopa = 0, vg = 0, vb = 0; };
-void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z);
+// tensors has been written (write observers), and for the same split of the n elements into [batch, z, rc] only.
+struct BnSource { const float *opa = nullptr, *g = nullptr, *b = nullptr; size_t n = 0, z = 0, rc = 0; unsigned long long vy = 0, vopa = 0, vg = 0, vb = 0; };
+void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z, size_t rc);
 // b of y = opa * g + b when y is still that, else nullptr
-const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n);
+const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n, size_t z, size_t rc);
 bool lz_enabled(DevCtx *c);
 
 }  // namespace eb

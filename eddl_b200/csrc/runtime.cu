@@ -264,20 +264,20 @@ void watch_forget(DevCtx *c, const void *p, size_t bytes) {
     for (uintptr_t k : gone) c->watch.erase(k);
 }
 
-void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z) {
+void bn_source_set(DevCtx *c, const float *y, const float *opa, const float *g, const float *b, size_t n, size_t z, size_t rc) {
     if (c->bn_sources.size() > 4096) c->bn_sources.clear();            // nets that are gone leave entries behind
     BnSource s;
-    s.opa = opa; s.g = g; s.b = b; s.n = n;
+    s.opa = opa; s.g = g; s.b = b; s.n = n; s.z = z; s.rc = rc;
     watch_add(c, y, n * sizeof(float)); watch_add(c, opa, n * sizeof(float)); watch_add(c, g, z * sizeof(float)); watch_add(c, b, z * sizeof(float));
     // overlapping ranges evict each other: read the versions once all four are registered (0 = not observed)
     s.vy = watch_version(c, y); s.vopa = watch_version(c, opa); s.vg = watch_version(c, g); s.vb = watch_version(c, b);
     c->bn_sources[y] = s;
 }
-const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n) {
+const float *bn_source_beta(DevCtx *c, const float *y, const float *opa, const float *g, size_t n, size_t z, size_t rc) {
     auto it = c->bn_sources.find(y);
     if (it == c->bn_sources.end()) return nullptr;
     const BnSource &s = it->second;
-    const bool same = s.opa == opa && s.g == g && s.n == n && s.vy && s.vopa && s.vg && s.vb && watch_version(c, y) == s.vy && watch_version(c, opa) == s.vopa &&
+    const bool same = s.opa == opa && s.g == g && s.n == n && s.z == z && s.rc == rc && s.vy && s.vopa && s.vg && s.vb && watch_version(c, y) == s.vy && watch_version(c, opa) == s.vopa &&
                       watch_version(c, g) == s.vg && watch_version(c, s.b) == s.vb;
     return same ? s.b : nullptr;
 }

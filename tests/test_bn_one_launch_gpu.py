@@ -93,6 +93,35 @@ def test_relu_backward_folded_in(lib, shape, own):
             np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("layout", [(8, 16, 1600), (16, 16, 800), (4, 32, 1600), (2, 8, 12800)], ids=lambda l: "x".join(map(str, l)))
+def test_relu_backward_folded_in_under_another_layout(lib, layout):
+    """bn_bwd over the buffers of an 8 x 32 x 800 forward pass, split into [batch, channels, pixels] in another way: what ReLU tests is the
+    tensor as it was written, not gamma and beta of the new channels."""
+    L = lib
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((8, 32, 20, 40)).astype(F)
+    g, b = rng.uniform(0.5, 1.5, 32).astype(F), rng.standard_normal(32).astype(F)
+    d, E = rng.standard_normal(x.shape).astype(F), x.size
+
+    def run(lazy):
+        L.call("set_option", b"lazy_zero", lazy)
+        try:
+            y, opa, r, gm, gv, me, va, dg, db = _forward(L, x, g, b)
+            dd, pd, gg, gb, m1, m2 = L.empty(x.shape), L.empty(x.shape), L.zeros((32,)), L.zeros((32,)), L.zeros((32,)), L.zeros((32,))
+            for a in (dd, pd):
+                L.call("fill", 0, a, E, 5.0); L.call("fill", 0, a, E, 0.0)
+            src, before = L.to_device(d), launches(L)        # kept alive: releasing it would run the record
+            L.call("relu_bwd", 0, src, y, dd, E)
+            L.call("bn_bwd", 0, *layout, dd, opa, pd, gg, gb, dg, va, m1, m2)
+            return launches(L) - before, [t.numpy() for t in (dd, pd, gg, gb, m1, m2)]
+        finally:
+            L.call("set_option", b"lazy_zero", 0)
+    (folded, got), (separate, want) = run(1), run(0)
+    assert folded == separate - 1                           # relu_bwd was taken over
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_relu_backward_with_copies(lib):
     """relu_bwd whose result is added into one or two zero deltas next (LAdd): one kernel, the bits of the separate calls; and a
     record that nothing takes over is run by the next call."""
