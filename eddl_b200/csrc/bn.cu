@@ -568,11 +568,11 @@ int launch_one(void (*kernel)(P...), bool &configured, const OnePlan &p, cudaStr
     return cuda_status(cudaGetLastError(), "gpu_batchnorm(one launch)");
 }
 
-// Training-mode forward in one launch; 1 = the channel does not fit (the caller takes the two-pass kernels).
+// Training-mode forward in one launch; kNotTaken = the caller takes the two-pass kernels.
 int fwd_one_launch(int dev, cudaStream_t st, unsigned b, unsigned z, unsigned rc, bool vec, const float *input, float *output, float *opa, float *global_mean, float *global_variance,
                    const float *affine_g, const float *affine_b, float *mean, float *variance, float epsilon, float momentum, float *relu_out) {
     OnePlan p;
-    if (!one_plan(z, b * rc, rc, 1, vec, p)) return 1;
+    if (!one_plan(z, b * rc, rc, 1, vec, p)) return kNotTaken;
     static bool configured[EDDLB200_MAX_DEVICES][2] = {};
     return launch_one(vec ? bn_fwd_one_kernel<true> : bn_fwd_one_kernel<false>, configured[dev][vec], p, st, input, output, opa, relu_out, global_mean, global_variance,
                       affine_g, affine_b, mean, variance, p.c, epsilon, momentum);
@@ -582,7 +582,7 @@ template <bool PD_ZERO, int MASK>
 int bwd_one_launch(int dev, cudaStream_t st, unsigned b, unsigned z, unsigned rc, bool vec, float *delta, const float *opa, float *pdelta, const float *src, const float *act,
                    const float *beta, float *gbn_g, float *gbn_b, const float *bn_g, const float *variance, float *mean1, float *mean2) {
     OnePlan p;
-    if (!one_plan(z, b * rc, rc, MASK == 1 ? 3 : 2, vec, p)) return 1;
+    if (!one_plan(z, b * rc, rc, MASK == 1 ? 3 : 2, vec, p)) return kNotTaken;
     static bool configured[EDDLB200_MAX_DEVICES][2] = {};
     return launch_one(vec ? bn_bwd_one_kernel<true, PD_ZERO, MASK> : bn_bwd_one_kernel<false, PD_ZERO, MASK>, configured[dev][vec], p, st, delta, opa, pdelta, src, act,
                       beta, gbn_g, gbn_b, bn_g, variance, mean1, mean2, p.c);
@@ -661,7 +661,7 @@ int eddlb200_bn_fwd(int dev, int b, int z, int rc, const float *input, float *ou
     if (trmode) {
         const int r = fwd_one_launch(dev, st, b, z, rc, vec, input, output, opa, global_mean, global_variance, affine_g, affine_b, mean, variance, epsilon, momentum, relu_out);
         if (r == 0) count_launch(cx);
-        if (r != 1) return r;
+        if (r != kNotTaken) return r;
         partial = (float2 *)scratch(cx, (size_t)z * S * sizeof(float2));
         if (!partial) return cudaErrorMemoryAllocation;
         fwd_two_pass(st, S, vec, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, z, rc, per, epsilon, momentum);
@@ -714,7 +714,7 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
                        : (mask == 0 ? bwd_one_launch<false, 0> : mask == 1 ? bwd_one_launch<false, 1> : bwd_one_launch<false, 2>);
     const int r = one(dev, st, b, z, rc, vec, delta, opa, pdelta, src, act, beta, gbn_g, gbn_b, bn_g, variance, mean1, mean2);
     if (r == 0) count_launch(cx);
-    if (r != 1) return r;
+    if (r != kNotTaken) return r;
     float2 *partial = (float2 *)scratch(cx, (size_t)z * S * sizeof(float2));
     if (!partial) return cudaErrorMemoryAllocation;
     auto two = pd_zero ? (mask == 0 ? bwd_two_pass<true, 0> : mask == 1 ? bwd_two_pass<true, 1> : bwd_two_pass<true, 2>)
@@ -815,7 +815,7 @@ extern "C" int eddlb200_bn_fwd_noalloc(int dev, int b, int z, int rc, const floa
     dim3 grid(z, S);
     if (trmode) {
         const int r = fwd_one_launch(dev, st, b, z, rc, vec, input, output, opa, global_mean, global_variance, affine_g, affine_b, mean, variance, epsilon, momentum, relu_out);
-        if (r != 1) return r;
+        if (r != kNotTaken) return r;
         fwd_two_pass(st, S, vec, input, output, opa, relu_out, partial, global_mean, global_variance, affine_g, affine_b, mean, variance, z, rc, per, epsilon, momentum);
     } else {
         if (vec) eb::launch(bn_fwd_apply_kernel<false, true>, grid, kBlock, 0, st, input, output, opa, relu_out, nullptr, global_mean, global_variance, affine_g, affine_b, mean, variance, per, w, epsilon, momentum);

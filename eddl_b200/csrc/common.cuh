@@ -188,6 +188,11 @@ int avg_settle(DevCtx *c, cudaStream_t st, const void *p, size_t bytes);
 
 namespace eb {
 
+// "This kernel does not take the call, use another one": an answer between the routes of an entry point, never returned to the caller.  Unlike
+// every status (CUDA errors are positive, 1 is cudaErrorInvalidValue; EDDLB200_E* are small and negative), so a launch that
+// fails is reported instead of being taken for a choice of route.
+constexpr int kNotTaken = -1000;
+
 __host__ __device__ inline size_t ceil_div(size_t a, size_t b) { return (a + b - 1) / b; }
 
 // Grid for a grid-stride elementwise kernel over `work` thread-items:

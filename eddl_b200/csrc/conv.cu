@@ -246,16 +246,16 @@ int eddlb200_conv2d_fwd(int dev, const float *x, const float *w, const float *bi
     EB_WRITES(y, (size_t)n * k * oh * ow * sizeof(float));
     ProfScope prof(cx, PROF_CONV_FWD, 2.0 * n * (double)k * c * kr * kc * oh * ow);
     if (tc_enabled()) {
-        if (int r = conv_tc_rs(cx, st, 0, g, x, w, y, bias, precision, false); r != 1) { g_conv_calls[dev][0]++; return r; }
+        if (int r = conv_tc_rs(cx, st, 0, g, x, w, y, bias, precision, false); r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
         const Dense1x1 d = dense_1x1(g, true);
         float *xs = d.on ? dense_buf(st, 0, (size_t)n * c * d.pitch * sizeof(float)) : nullptr;
         if (xs) {
             if (int r = gather_planes(cx, st, x, xs, (size_t)n * c, ih, iw, sr, sc, oh, ow, d.pitch)) return r;
             int r = conv_tc_fwd(cx, st, d.g, xs, w, bias, y, precision);
-            if (r != 1) { g_conv_calls[dev][0]++; return r; }
+            if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
         }
         int r = conv_tc_fwd(cx, st, g, x, w, bias, y, precision);
-        if (r != 1) { g_conv_calls[dev][0]++; return r; }
+        if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
     }
     g_conv_calls[dev][1]++;
     return conv_simt_fwd(cx, st, g, x, w, bias, y);
@@ -276,7 +276,7 @@ int eddlb200_conv2d_bwd_data(int dev, const float *dy, const float *w, float *dx
     if (lz_any(cx)) { int status = 0; dx_zero = lz_take(cx, st, dx, dx_elems * sizeof(float), &status); if (status) return status; }
     ProfScope prof(cx, PROF_CONV_BWD_DATA, 2.0 * n * (double)k * c * kr * kc * oh * ow);
     if (tc_enabled()) {
-        if (int r = conv_tc_rs(cx, st, 1, g, dy, w, dx, nullptr, precision, dx_zero); r != 1) { g_conv_calls[dev][0]++; return r; }
+        if (int r = conv_tc_rs(cx, st, 1, g, dy, w, dx, nullptr, precision, dx_zero); r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
         const Dense1x1 d = dense_1x1(g, true);
         float *dense = d.on ? dense_buf(st, 2, (size_t)n * c * d.pitch * sizeof(float)) : nullptr;
         if (dense) {
@@ -291,10 +291,10 @@ int eddlb200_conv2d_bwd_data(int dev, const float *dy, const float *w, float *dx
                 g_conv_calls[dev][0]++;
                 return 0;
             }
-            if (r != 1) return r;
+            if (r != kNotTaken) return r;
         }
         int r = conv_tc_bwd_data(cx, st, g, dy, w, dx, precision, dx_zero);
-        if (r != 1) { g_conv_calls[dev][0]++; return r; }
+        if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
     }
     g_conv_calls[dev][1]++;
     if (dx_zero) { if (int r = launch_zero_fill(cx, st, dx, dx_elems)) return r; }     // the FMA kernel adds into dx
@@ -333,7 +333,7 @@ int eddlb200_conv2d_bwd_weight(int dev, const float *x, const float *dy, float *
             if (int r = gather_planes(cx, st, dy, dys, (size_t)n * k, oh, ow, 1, 1, oh, wp, oh * wp, ow)) return r;
             const ConvGeom gp{n, c, ih, wp, k, 3, 3, oh, wp, 1, 1, 1, 1};
             int r = conv_tc_bwd_weight(cx, st, gp, xs, dys, gw, precision, gw_zero);
-            if (r != 1) { g_conv_calls[dev][0]++; return r; }
+            if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
         }
     }
     if (tc_enabled()) {
@@ -344,10 +344,10 @@ int eddlb200_conv2d_bwd_weight(int dev, const float *x, const float *dy, float *
             if (int r = gather_planes(cx, st, x, xs, (size_t)n * c, ih, iw, sr, sc, oh, ow, d.pitch)) return r;
             if (dys) { if (int r = gather_planes(cx, st, dy, dys, (size_t)n * k, oh, ow, 1, 1, oh, ow, d.pitch)) return r; }
             int r = conv_tc_bwd_weight(cx, st, d.g, xs, dys ? dys : dy, gw, precision, gw_zero);
-            if (r != 1) { g_conv_calls[dev][0]++; return r; }
+            if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
         }
         int r = conv_tc_bwd_weight(cx, st, g, x, dy, gw, precision, gw_zero);
-        if (r != 1) { g_conv_calls[dev][0]++; return r; }
+        if (r != kNotTaken) { g_conv_calls[dev][0]++; return r; }
     }
     g_conv_calls[dev][1]++;
     if (gw_zero) { if (int r = launch_zero_fill(cx, st, gw, gw_elems)) return r; }     // the FMA path adds into gw

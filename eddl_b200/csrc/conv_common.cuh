@@ -16,7 +16,7 @@ int conv_simt_fwd(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x
 int conv_simt_bwd_data(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *dy, const float *w, float *dx);
 int conv_simt_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *dy, float *gw);
 
-// Tensor-core implicit GEMM (conv_tc.cu).  Each returns 1 when the shape is outside what
+// Tensor-core implicit GEMM (conv_tc.cu).  Each returns kNotTaken when the shape is outside what
 // the kernel takes (the caller then uses the FMA path), 0 on success, or an error code.
 int conv_tc_fwd(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *w, const float *bias, float *y, int precision);
 // dx_zero: dx is known to hold zeros (the caller took over a deferred zero fill of it), so the result may be stored
@@ -26,7 +26,7 @@ int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const floa
 bool conv_tc_allowed();          // false while eddlb200_set_option("conv_path", 1) / EDDL_B200_CONV=simt forces the fp32 FMA kernels
 int conv_tc_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool gw_zero);
 
-// Forward (mode 0: src = x, out = y) and backward-data (mode 1: src = dy, out = dx) on pairs of CTAs (conv_rs.cuh); 1 = not taken.
+// Forward (mode 0: src = x, out = y) and backward-data (mode 1: src = dy, out = dx) on pairs of CTAs (conv_rs.cuh); kNotTaken = another kernel's layer.
 int conv_tc_rs(DevCtx *cx, cudaStream_t st, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias, int precision, bool out_zero);
 // 1 (default): that kernel runs the layers it is the faster one for; 2: every layer it fits; 0: none.
 int conv_tc_set_rs(int level);

@@ -1671,17 +1671,17 @@ bool conv_rs_plan(const ConvGeom &g, int mode, int precision, RsPlan &plan) {
 
 int g_conv_rs = 1;             // eddlb200_set_option("conv_pairs", 0 off / 1 where it is the faster kernel / 2 wherever it fits)
 
-// mode 0 forward, 1 backward-data; 1 = not taken
+// mode 0 forward, 1 backward-data
 int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias,
            int precision, bool out_zero) {
-    if (!g_conv_rs) return 1;
+    if (!g_conv_rs) return kNotTaken;
     RsPlan plan;
-    if (!conv_rs_plan(g, mode, precision, plan)) return 1;
+    if (!conv_rs_plan(g, mode, precision, plan)) return kNotTaken;
     RsParams &P = plan.P;
     if (g_conv_rs < 2) {
         // Layers of a few channels stay on the gather kernels (a K-block here is 32 channels of one tap), layers of a few dx channels
         // with their GEMM route; otherwise the smaller estimate wins.
-        if (P.C < 16 || P.K < 8 || (mode == 1 && g.c <= 8)) return 1;
+        if (P.C < 16 || P.K < 8 || (mode == 1 && g.c <= 8)) return kNotTaken;
         const bool dense = g.sr == 1 && g.sc == 1;
         double other = gather_layer_us(g, mode);
         if (mode == 1 && !dense) other *= 2.0;                            // one launch per parity class, none of them split
@@ -1692,7 +1692,7 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
                                         (dense ? 0.0 : 6.0 + 8.0 * g.n * (mode == 0 ? g.c : g.c * g.sr * g.sc) * (double)pq / 5.0e6));
         if (dense && g.kr == 3 && g.kc == 3 && g.pt == 1 && g.pl == 1 && g.iw == g.ow && g.ih == g.oh && pq % 4 == 0 && pq >= 64 && g.iw <= 61 && P.C >= 32 && P.K >= 32)
             other = std::min(other, tma_fed_us((long long)g.n * ((pq + BM - 1) / BM) * tiles_n, 9 * P.cgs));
-        if (plan.us > 0.95 * other) return 1;
+        if (plan.us > 0.95 * other) return kNotTaken;
     }
     const int planes = precision == 1 ? 1 : 2;
     if (mode == 1 && out_zero) {
@@ -1709,7 +1709,7 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
     auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     const size_t o_kA = carve((size_t)T.K_pad * 8), o_rowB = carve((size_t)T.N_total * 4), o_kB = carve((size_t)T.K_pad * 4), o_kC = carve((size_t)T.K_pad * 4);
     tb = cached_table(dev, table_key(T), off, build);
-    if (!tb) return 1;
+    if (!tb) return kNotTaken;
     T.rowA = nullptr; T.outM = nullptr; T.kA = (int2 *)(tb + o_kA); T.rowB = (int *)(tb + o_rowB); T.kB = (int *)(tb + o_kB); T.kC = (int *)(tb + o_kC);
     if (build) {
         eb::launch(build_tables_kernel, grid_for((size_t)T.K_pad + T.N_total, 256), 256, 0, st, T);
@@ -1732,9 +1732,9 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
         }
     }
     if (entry && entry->packed == img) {
-        if (!entry->has_map) { if (!encode_rows_map(&entry->map, img, image_rows, plan.bn / 2)) return 1; entry->has_map = true; }
+        if (!entry->has_map) { if (!encode_rows_map(&entry->map, img, image_rows, plan.bn / 2)) return kNotTaken; entry->has_map = true; }
         P.mapB = entry->map;
-    } else if (!encode_rows_map(&P.mapB, img, image_rows, plan.bn / 2)) return 1;
+    } else if (!encode_rows_map(&P.mapB, img, image_rows, plan.bn / 2)) return kNotTaken;
     if (int r = status_word(dev, st)) return r;
     P.status = g_status[dev];
     P.src = src; P.out = out; P.bias = mode == 0 ? bias : nullptr;
@@ -1775,11 +1775,11 @@ int combine_splits(DevCtx *cx, cudaStream_t st, const float *part, float *out, s
     return 0;
 }
 
-// Backward-weight on CTA pairs (conv_wg.cuh) of a layer that the TMA-fed kernels take (slab: 3x3 "same", otherwise 1x1 dense); 1 = the
-// kernel on single CTAs is the faster one.  A pair has twice the rows of a CTA, so a layer with few rows leaves half of it empty,
+// Backward-weight on CTA pairs (conv_wg.cuh) of a layer that the TMA-fed kernels take (slab: 3x3 "same", otherwise 1x1 dense);
+// kNotTaken where the kernel on single CTAs is the faster one.  A pair has twice the rows of a CTA, so a layer with few rows leaves half of it empty,
 // and half as many units to fill: both estimates are made with the splits that each would choose.
 int run_wg(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool slab, bool gw_zero) {
-    if (!g_conv_rs) return 1;
+    if (!g_conv_rs) return kNotTaken;
     const int pq = g.oh * g.ow, chunks = (pq + 31) / 32, kblocks = g.n * chunks, sp_min = (kblocks + kMaxChainBlocks - 1) / kMaxChainBlocks;
     const size_t out_total = (size_t)g.k * g.c * g.kr * g.kc;
     auto kblock_us = [&](int bn, bool pairs) {
@@ -1799,12 +1799,12 @@ int run_wg(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g, const float 
     };
     Plan p = plan(false, true);
     if (!slab) { const Plan q = plan(true, true); if (q.c.us < 0.98 * p.c.us) p = q; }
-    if (g_conv_rs < 2 && p.c.us > 0.97 * plan(false, false).c.us) return 1;
+    if (g_conv_rs < 2 && p.c.us > 0.97 * plan(false, false).c.us) return kNotTaken;
     WgParams P{};
     const float *a = p.swap ? dy : x, *b = p.swap ? x : dy;
     const int ca = p.swap ? g.k : g.c, cb = p.swap ? g.c : g.k;
     const bool maps = slab ? encode_plane_map(&P.mapA, a, pq, ca, g.n, WS_SLAB_CH, false, WS_SLAB_PX) : encode_plane_map(&P.mapA, a, pq, ca, g.n, BM, true);
-    if (!maps || !encode_plane_map(&P.mapB, b, pq, cb, g.n, p.bn / 2, true)) return 1;
+    if (!maps || !encode_plane_map(&P.mapB, b, pq, cb, g.n, p.bn / 2, true)) return kNotTaken;
     const int kbs = (kblocks + p.c.splits - 1) / p.c.splits, splits = (kblocks + kbs - 1) / kbs;
     if (int r = status_word(dev, st)) return r;
     float *part = splits > 1 ? (float *)scratch(cx, out_total * splits * sizeof(float)) : nullptr;
@@ -1857,7 +1857,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
     bool wtma = planes_dense && g_conv_wtma > 0 && g.oh * g.ow >= 32 && g.c >= 32 && g.k >= 32;
     int w_bn = 0;
     if (wtma) {
-        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, false, out_zero); r != 1) return r;
+        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, false, out_zero); r != kNotTaken) return r;
         w_bn = T.N_total <= 32 ? 32 : (T.N_total <= 64 ? 64 : 128);
         P.chunks_per_image = w_chunks; P.images = g.n; P.raw_hi = g_conv_wtma > 1;
         if (!encode_plane_map(&P.mapA, srcA, g.oh * g.ow, g.c, g.n, BM, true) || !encode_plane_map(&P.mapOut, srcB, g.oh * g.ow, g.k, g.n, w_bn, true)) wtma = false;
@@ -1870,7 +1870,7 @@ int run_one(DevCtx *cx, cudaStream_t st, int dev, TableArgs T, TcParams P, const
                  g.ih == g.oh && g.iw == g.ow && g.iw >= 3 && 2 * (g.iw + 1) + BK + 3 <= WS_SLAB_PX && (g.oh * g.ow) % 4 == 0 && g.oh * g.ow >= 32 &&
                  g.c >= WS_CH && g.k >= 32 && aligned16(srcA) && aligned16(srcB);
     if (wslab) {
-        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, true, out_zero); r != 1) return r;
+        if (int r = run_wg(cx, st, dev, g, srcA, srcB, out, precision, true, out_zero); r != kNotTaken) return r;
         const int ws_bn = T.N_total <= 32 ? 32 : (T.N_total <= 64 ? 64 : 128);
         P.chunks_per_image = w_chunks; P.images = g.n; P.raw_hi = g_conv_wtma > 1; P.img_w = g.iw; P.plane_px = g.oh * g.ow;
         if (!encode_plane_map(&P.mapA, srcA, g.oh * g.ow, g.c, g.n, WS_SLAB_CH, false, WS_SLAB_PX) ||
@@ -2086,7 +2086,7 @@ int run_small_c_bwd_data(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g
         cudaStreamSynchronize(st);
         if (tbuf[dev]) cudaFree(tbuf[dev]);
         tbuf[dev] = nullptr; tcap[dev] = 0;
-        if (cudaMalloc((void **)&tbuf[dev], t_elems * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return 1; }
+        if (cudaMalloc((void **)&tbuf[dev], t_elems * sizeof(float)) != cudaSuccess) { cudaGetLastError(); return kNotTaken; }
         tcap[dev] = t_elems;
     }
     // The GEMM is a 1x1 stride-1 convolution of dy ([image][filter][pixel], the filters as input channels) with the weights
@@ -2108,8 +2108,8 @@ int run_small_c_bwd_data(DevCtx *cx, cudaStream_t st, int dev, const ConvGeom &g
         if (watch_any(cx)) note_write(cx, wt[dev], w_elems * sizeof(float));       // the packed image of the copy is stale now
         // the plane as one row of pq pixels: a 1x1 layer does not care about its two-dimensional shape
         const ConvGeom g1{g.n, g.k, 1, pq, g.c * rs, 1, 1, 1, pq, 1, 1, 0, 0};
-        const int r = pq < 16000 ? run(cx, st, dev, 0, g1, dy, wt[dev], tbuf[dev], nullptr, precision) : 1;
-        if (r != 0 && r != 1) return r;
+        const int r = pq < 16000 ? run(cx, st, dev, 0, g1, dy, wt[dev], tbuf[dev], nullptr, precision) : kNotTaken;
+        if (r != 0 && r != kNotTaken) return r;
         dense = r == 0;
     }
     if (!dense) {
@@ -2134,13 +2134,13 @@ bool fits(const ConvGeom &g) {
 namespace eb {
 
 int conv_tc_fwd(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *w, const float *bias, float *y, int precision) {
-    if (!fits(g)) return 1;
+    if (!fits(g)) return kNotTaken;
     int dev = 0; cudaGetDevice(&dev);
     return run(cx, st, dev, 0, g, x, w, y, bias, precision);
 }
 
 int conv_tc_bwd_data(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *dy, const float *w, float *dx, int precision, bool dx_zero) {
-    if (!fits(g)) return 1;
+    if (!fits(g)) return kNotTaken;
     int dev = 0; cudaGetDevice(&dev);
     const bool small_c = g.c <= 8 && (size_t)g.n * g.c * g.kr * g.kc * g.oh * g.ow < (size_t(1) << 29);
     if (dx_zero && (small_c || g.sr != 1 || g.sc != 1)) {
@@ -2150,22 +2150,22 @@ int conv_tc_bwd_data(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float
     }
     if (g.c <= 8 && (size_t)g.n * g.c * g.kr * g.kc * g.oh * g.ow < (size_t(1) << 29)) {
         const int r = run_small_c_bwd_data(cx, st, dev, g, dy, w, dx, precision);
-        if (r != 1) return r;
+        if (r != kNotTaken) return r;
     }
     return run(cx, st, dev, 1, g, dy, w, dx, nullptr, precision, dx_zero);
 }
 
 int conv_tc_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool gw_zero) {
-    if (!fits(g)) return 1;
+    if (!fits(g)) return kNotTaken;
     int dev = 0; cudaGetDevice(&dev);
     return run(cx, st, dev, 2, g, x, dy, gw, nullptr, precision, gw_zero);
 }
 
 // C[m x n] (row-major) = op(A) op(B), += when inc_c == 1, written into known zeros when inc_c == 2: the dense layers' GEMMs
 // (Tensor::mult2D, src/tensor/tensor_math.cpp) on the same kernel, as a "convolution" whose rows are the rows of op(A).
-// 1 = not taken (the caller falls back to the fp32 FMA GEMM).
+// kNotTaken = the caller runs the fp32 FMA GEMM.
 int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const float *b, int tb, float *c, int inc_c, int m, int n, int k, int precision) {
-    if ((long long)m * k >= 0x7fffffffLL || (long long)n * k >= 0x7fffffffLL || (long long)m * n >= 0x7fffffffLL) return 1;
+    if ((long long)m * k >= 0x7fffffffLL || (long long)n * k >= 0x7fffffffLL || (long long)m * n >= 0x7fffffffLL) return kNotTaken;
     int dev = 0; cudaGetDevice(&dev);
     TableArgs T{};
     T.g = ConvGeom{m, k, ta ? 1 : 0, tb ? 1 : 0, n, 1, 1, 1, 1, 1, 1, 0, 0};
@@ -2176,7 +2176,7 @@ int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const floa
 }
 
 int conv_tc_rs(DevCtx *cx, cudaStream_t st, int mode, const ConvGeom &g, const float *src, const float *w, float *out, const float *bias, int precision, bool out_zero) {
-    if (!fits(g)) return 1;
+    if (!fits(g)) return kNotTaken;
     int dev = 0; cudaGetDevice(&dev);
     return run_rs(cx, st, dev, mode, g, src, w, out, bias, precision, out_zero);
 }

@@ -185,7 +185,7 @@ int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, flo
     // (64 x 1000 x 2048 for ResNet-50's classifier: 29 -> 11 us), and a library forced to the FMA path stays here.
     if (conv_tc_allowed() && k >= 32 && (double)m * n * k >= 536870912.0) {
         const int r = conv_tc_gemm(cx, st, a, ta, b, tb, c, inc_c, m, n, k, 0);
-        if (r != 1) return r;
+        if (r != kNotTaken) return r;
     }
     // k slices: two blocks per SM where the tiles alone do not give them, slices of at least 64 (two k steps)
     const long long tiles = (long long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);

@@ -80,6 +80,7 @@ int set_error(int code, const char *fmt, ...) {
 
 int cuda_status(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return 0;
+    cudaGetLastError();             // reported here: the next call's launch check must not find it again
     set_error((int)e, "[CUDA ERROR]: %s (%d) raised in %s", cudaGetErrorString(e), (int)e, what);
     return (int)e;
 }

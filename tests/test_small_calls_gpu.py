@@ -96,3 +96,32 @@ def test_multi_tensor_tables_are_told_apart(lib):
             wp, wm = orc.sgd_step(p, g, m, 0.1, 0.9)
             np.testing.assert_array_equal(dp.numpy(), wp); np.testing.assert_array_equal(dm.numpy(), wm)
             lists[i] = (wp, g, wm, dp, dg, dm)
+
+
+def test_a_reported_error_changes_nothing_for_the_calls_after_it(lib):
+    """A copy that CUDA refuses (cudaErrorInvalidValue, the value 1) is reported once.  The kernels launched next run once, whatever
+    route they take: statistics and deltas that are read, changed and written back show a second run."""
+    from eddl_b200 import capi
+    rng = np.random.default_rng(3)
+    n, z, h = 8, 64, 14
+    x, d, x0 = (rng.standard_normal((n, z, h, h)).astype(F) for _ in range(3))
+    w, g, b = rng.standard_normal((z, z, 3, 3)).astype(F), rng.uniform(0.5, 1.5, z).astype(F), rng.standard_normal(z).astype(F)
+
+    def run(refused):
+        def after():
+            if refused:
+                with pytest.raises(capi.Error):
+                    lib.call("memcpy_h2d", 0, None, x.ctypes.data_as(ctypes.c_void_p), 64)
+        dx, dd, dg, db, dw = (lib.to_device(a) for a in (x, d, g, b, w))
+        y, opa, me, va, m1, m2 = lib.empty(x.shape), lib.empty(x.shape), lib.empty((z,)), lib.empty((z,)), lib.empty((z,)), lib.empty((z,))
+        gm, gv, gg, gb = lib.zeros((z,)), lib.zeros((z,)), lib.zeros((z,)), lib.zeros((z,))
+        pd, cx, gw, c = lib.to_device(x0), lib.to_device(x0), lib.to_device(w), lib.to_device(x0[0, 0])
+        geo = (n, z, h, h, z, 3, 3, h, h, 1, 1, 1, 1, 0)
+        after(); lib.call("bn_fwd", 0, n, z, h * h, dx, y, opa, gm, gv, dg, db, me, va, 1, 1e-3, 0.9, None)
+        after(); lib.call("conv2d_bwd_data", 0, dd, dw, cx, *geo)
+        after(); lib.call("conv2d_bwd_weight", 0, dx, dd, gw, None, *geo)
+        after(); lib.call("bn_bwd", 0, n, z, h * h, dd, opa, pd, gg, gb, dg, va, m1, m2)
+        after(); lib.call("mult2d", 0, dx, 0, dx, 0, c, 1, h, h, h)
+        return [t.numpy() for t in (y, gm, gv, cx, gw, dd, pd, gg, gb, c)]
+    for got, want in zip(run(True), run(False)):
+        np.testing.assert_array_equal(got, want)
