@@ -16,6 +16,7 @@
 // backward 16 (delta, opa; delta *= gamma in place as in the reference, parent delta);
 // two-pass +4 and +8.
 #include <cooperative_groups.h>
+#include <atomic>
 #include <mutex>
 #include "common.cuh"
 
@@ -551,19 +552,31 @@ bool one_plan(unsigned z, unsigned per, unsigned rc, int tensors, bool vec, OneP
     if ((size_t)z * per * 4 > (size_t)8 << 20 && (cs > 1 || tensors > 1)) return false;
     return true;
 }
+// What a kernel has been set up for on one device.
+struct OneSetup { std::atomic<bool> attributes{false}; std::atomic<unsigned> wide_smem{0}; };        // wide_smem: shared memory known to fit clusters of 16
+// kNotTaken where the device cannot hold a cluster of this size (more than eight blocks are not guaranteed: a 16-block cluster needs
+// that many SMs of one cluster group free of other limits); a launch that fails for any other reason is an error.
 template <typename... P, typename... A>
-int launch_one(void (*kernel)(P...), bool &configured, const OnePlan &p, cudaStream_t st, A &&...args) {
-    if (!configured) {
+int launch_one(void (*kernel)(P...), OneSetup &setup, const OnePlan &p, cudaStream_t st, A &&...args) {
+    if (!setup.attributes) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return cuda_status(e, "gpu_batchnorm(attributes)");
-        configured = true;
+        setup.attributes = true;
     }
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = p.c.csize; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = p.c.csize; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.blocks); cfg.blockDim = dim3(p.threads); cfg.dynamicSmemBytes = p.smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 2;
+    if (p.c.csize > 8 && p.smem > setup.wide_smem) {
+        cudaLaunchConfig_t query = cfg;
+        query.blockDim = dim3(kOneBlock); query.numAttrs = 1;              // the largest block: what fits it fits the smaller ones
+        int clusters = 0;
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &query);
+        if (e != cudaSuccess || clusters < 1) { cudaGetLastError(); return kNotTaken; }
+        setup.wide_smem = p.smem;
+    }
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
     return cuda_status(cudaGetLastError(), "gpu_batchnorm(one launch)");
 }
@@ -573,8 +586,8 @@ int fwd_one_launch(int dev, cudaStream_t st, unsigned b, unsigned z, unsigned rc
                    const float *affine_g, const float *affine_b, float *mean, float *variance, float epsilon, float momentum, float *relu_out) {
     OnePlan p;
     if (!one_plan(z, b * rc, rc, 1, vec, p)) return kNotTaken;
-    static bool configured[EDDLB200_MAX_DEVICES][2] = {};
-    return launch_one(vec ? bn_fwd_one_kernel<true> : bn_fwd_one_kernel<false>, configured[dev][vec], p, st, input, output, opa, relu_out, global_mean, global_variance,
+    static OneSetup setup[EDDLB200_MAX_DEVICES][2];
+    return launch_one(vec ? bn_fwd_one_kernel<true> : bn_fwd_one_kernel<false>, setup[dev][vec], p, st, input, output, opa, relu_out, global_mean, global_variance,
                       affine_g, affine_b, mean, variance, p.c, epsilon, momentum);
 }
 
@@ -583,8 +596,8 @@ int bwd_one_launch(int dev, cudaStream_t st, unsigned b, unsigned z, unsigned rc
                    const float *beta, float *gbn_g, float *gbn_b, const float *bn_g, const float *variance, float *mean1, float *mean2) {
     OnePlan p;
     if (!one_plan(z, b * rc, rc, MASK == 1 ? 3 : 2, vec, p)) return kNotTaken;
-    static bool configured[EDDLB200_MAX_DEVICES][2] = {};
-    return launch_one(vec ? bn_bwd_one_kernel<true, PD_ZERO, MASK> : bn_bwd_one_kernel<false, PD_ZERO, MASK>, configured[dev][vec], p, st, delta, opa, pdelta, src, act,
+    static OneSetup setup[EDDLB200_MAX_DEVICES][2];
+    return launch_one(vec ? bn_bwd_one_kernel<true, PD_ZERO, MASK> : bn_bwd_one_kernel<false, PD_ZERO, MASK>, setup[dev][vec], p, st, delta, opa, pdelta, src, act,
                       beta, gbn_g, gbn_b, bn_g, variance, mean1, mean2, p.c);
 }
 

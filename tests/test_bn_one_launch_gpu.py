@@ -9,7 +9,7 @@ from oracle import eddl_oracle as orc
 
 pytestmark = pytest.mark.gpu
 F = np.float32
-SHAPES = [(1, 1, 1, 1), (2, 3, 1, 2), (5, 7, 7, 7), (3, 33, 2, 2), (4, 5, 9, 13), (64, 2, 28, 28), (3, 300, 10, 10), (16, 3, 64, 64), (2, 4, 113, 115), (129, 2, 100, 36), (40, 2, 256, 256)]
+SHAPES = [(1, 1, 1, 1), (2, 3, 1, 2), (5, 7, 7, 7), (3, 33, 2, 2), (4, 5, 9, 13), (64, 2, 28, 28), (3, 300, 10, 10), (16, 3, 64, 64), (2, 4, 113, 115), (129, 2, 100, 36), (40, 2, 256, 256), (112, 2, 64, 64)]
 
 
 def launches(L):
@@ -55,6 +55,17 @@ def test_forward_and_backward(lib, shape):
     np.testing.assert_array_equal(dd.numpy(), (delta * g[None, :, None, None]).astype(F))
     a = (m1.numpy()[None, :, None, None] * o).astype(F) + m2.numpy()[None, :, None, None]
     np.testing.assert_array_equal(pd.numpy(), pd0 + ((dd.numpy() - a.astype(F)).astype(F) / s).astype(F))
+
+
+def test_the_widest_share_is_one_launch(lib):
+    """Sixteen blocks with all the shared memory that a share may have: the device is asked whether it holds such a cluster, and it does."""
+    L = lib
+    x = np.random.default_rng(6).standard_normal((112, 2, 64, 64)).astype(F)
+    dx, y, opa, ones, zeros, me, va = L.to_device(x), L.empty(x.shape), L.empty(x.shape), L.to_device(np.ones(2, F)), L.zeros((2,)), L.empty((2,)), L.empty((2,))
+    for _ in range(2):
+        before = launches(L)
+        L.call("bn_fwd", 0, 112, 2, 4096, dx, y, opa, zeros, ones, ones, zeros, me, va, 1, 1e-3, 0.0, None)
+        assert launches(L) == before + 1
 
 
 @pytest.mark.parametrize("shape", [(64, 4, 28, 28), (30, 50, 7, 7), (8, 2, 256, 256), (64, 300, 2, 2)], ids=lambda s: "x".join(map(str, s)))
