@@ -42,6 +42,7 @@ struct TensorRef { float *p; const float *g; float *m; unsigned long long n; };
 
 // One block-chunk table entry per `chunk` elements: (tensor, offset).
 struct Chunk { unsigned tensor; unsigned offset_k; };   // offset in units of `chunk` elements
+constexpr size_t kMaxElements = size_t(1) << 40;        // 4 TB of parameters: no device holds that
 // 16K elements per chunk keep the table short; parameter sets that would then give an SM fewer than its eight resident blocks
 // are cut four times finer (2.9 M parameters with Adam: 35 -> 20 us)
 inline unsigned chunk_for(size_t total) { return total < (size_t)16384 * EDDLB200_NUM_SMS * 8 ? 4096u : 16384u; }
@@ -177,12 +178,14 @@ int eddlb200_sgd_momentum_multi(int dev, float *const *p, const float *const *g,
     if (ntensors == 0) return 0;
     std::vector<TensorRef> refs; std::vector<Chunk> chunks;
     size_t elements = 0;
-    for (int i = 0; i < ntensors; i++) elements += sizes[i];
+    for (int i = 0; i < ntensors; i++) {
+        EB_REQUIRE(sizes[i] == 0 || (p[i] && g[i] && m[i]), "sgd_multi");
+        EB_REQUIRE(sizes[i] < kMaxElements && (elements += sizes[i]) < kMaxElements, "sgd_multi");        // nothing is reserved for sizes that cannot be
+    }
     const unsigned chunk = chunk_for(elements);
     refs.reserve(ntensors); chunks.reserve(elements / chunk + ntensors);
     for (int i = 0; i < ntensors; i++) {
         if (sizes[i] == 0) continue;
-        EB_REQUIRE(p[i] && g[i] && m[i], "sgd_multi");
         EB_MODIFIES(p[i], sizes[i] * sizeof(float)); EB_READS(g[i], sizes[i] * sizeof(float)); EB_MODIFIES(m[i], sizes[i] * sizeof(float));
         refs.push_back(TensorRef{p[i], g[i], m[i], (unsigned long long)sizes[i]});
         const size_t nch = ceil_div(sizes[i], (size_t)chunk);
@@ -222,12 +225,14 @@ int eddlb200_adam_multi(int dev, float *const *p, float *const *g, float *const 
     if (ntensors == 0) return 0;
     std::vector<AdamRef> refs; std::vector<Chunk> chunks;
     size_t elements = 0;
-    for (int i = 0; i < ntensors; i++) elements += sizes[i];
+    for (int i = 0; i < ntensors; i++) {
+        EB_REQUIRE(sizes[i] == 0 || (p[i] && g[i] && m[i] && v[i]), "adam_multi");
+        EB_REQUIRE(sizes[i] < kMaxElements && (elements += sizes[i]) < kMaxElements, "adam_multi");        // nothing is reserved for sizes that cannot be
+    }
     const unsigned chunk = chunk_for(elements);
     refs.reserve(ntensors); chunks.reserve(elements / chunk + ntensors);
     for (int i = 0; i < ntensors; i++) {
         if (sizes[i] == 0) continue;
-        EB_REQUIRE(p[i] && g[i] && m[i] && v[i], "adam_multi");
         const size_t bytes = sizes[i] * sizeof(float);
         EB_MODIFIES(p[i], bytes); EB_MODIFIES(g[i], bytes); EB_MODIFIES(m[i], bytes); EB_MODIFIES(v[i], bytes);
         refs.push_back(AdamRef{p[i], g[i], m[i], v[i], (unsigned long long)sizes[i]});

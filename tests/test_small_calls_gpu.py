@@ -98,6 +98,24 @@ def test_multi_tensor_tables_are_told_apart(lib):
             lists[i] = (wp, g, wm, dp, dg, dm)
 
 
+@pytest.mark.parametrize("name,tensors", [("sgd_momentum_multi", 3), ("adam_multi", 4)])
+def test_multi_tensor_calls_refuse_what_cannot_be(lib, name, tensors):
+    """A list with a missing tensor or a size that no device holds is an error of the call, whatever its other sizes say, and no tensor
+    of the list has been touched."""
+    from eddl_b200 import capi
+    more = (0.1, 0.9) if tensors == 3 else (0.1, 0.9, 0.999, 1e-8, 1)
+    good = [lib.to_device(np.full(8, 1 + i, F)) for i in range(tensors)]
+    for missing in range(-1, tensors):
+        for size in (7, 2 ** 40, 2 ** 62, 2 ** 64 - 8):
+            if missing < 0 and size == 7:
+                continue
+            lists = [(ctypes.c_void_p * 2)(a.addr, None if i == missing else a.addr) for i, a in enumerate(good)]
+            with pytest.raises(capi.Error):
+                lib.call(name, 0, *lists, (ctypes.c_size_t * 2)(8, size), 2, *more)
+    for i, a in enumerate(good):
+        np.testing.assert_array_equal(a.numpy(), np.full(8, 1 + i, F))
+
+
 def test_a_reported_error_changes_nothing_for_the_calls_after_it(lib):
     """A copy that CUDA refuses (cudaErrorInvalidValue, the value 1) is reported once.  The kernels launched next run once, whatever
     route they take: statistics and deltas that are read, changed and written back show a second run."""
