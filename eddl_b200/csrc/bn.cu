@@ -698,7 +698,14 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
     int mask = 0;
     if (pend_copy_active(cx)) {
         PendCopy &p = pend_copy(cx);
-        if (p.kind == 4 && p.dst == delta && p.n == elements && p.src != pdelta && p.src2 != pdelta && pdelta != delta) {
+        // what the fold reads after the call has begun to write: the two inputs of the ReLU backward pass, which a caller may give
+        // up (and use again for an output) once that pass has been called
+        bool apart = pdelta != delta;
+        for (const float *in : {p.src, p.src2}) {
+            const size_t tb = elements * sizeof(float), zb = (size_t)z * sizeof(float);
+            apart = apart && !overlap(in, tb, pdelta, tb) && !overlap(in, tb, gbn_g, zb) && !overlap(in, tb, gbn_b, zb) && !overlap(in, tb, mean1, zb) && !overlap(in, tb, mean2, zb);
+        }
+        if (p.kind == 4 && p.dst == delta && p.n == elements && apart) {
             // the ReLU backward pass that makes this delta is still on record: it is folded in
             p.active = false;
             src = p.src; act = p.src2;

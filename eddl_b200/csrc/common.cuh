@@ -205,6 +205,10 @@ inline int grid_for(size_t work_items, int block, int max_blocks_per_sm = 8) {
     return (int)blocks;
 }
 
+inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+    return a && b && (uintptr_t)a < (uintptr_t)b + b_bytes && (uintptr_t)b < (uintptr_t)a + a_bytes;
+}
+
 __host__ __device__ inline bool aligned16(const void *p) { return (((uintptr_t)p) & 15u) == 0; }
 
 #ifdef __CUDACC__

@@ -380,8 +380,8 @@ int eddlb200_axpby(int dev, float sca, const float *a, float scb, const float *b
             if (lz_take(cx, st, c, n * sizeof(float), &status)) { p.kind = 3; p.dst2 = c; return 0; }
             if (status) return status;
         }
-        if ((p.kind == 4 || (p.kind == 5 && !p.dst3)) && !inc_c && c && c == b && a == p.dst && n == p.n && c != p.dst && c != p.dst2 && c != p.src && c != p.src2 && lz_any(cx) &&
-            (p.kind == 4 || (sca == p.sa && scb == p.sb))) {
+        if ((p.kind == 4 || (p.kind == 5 && !p.dst3)) && !inc_c && c && c == b && a == p.dst && n == p.n && c != p.dst && c != p.dst2 && lz_any(cx) &&
+            !overlap(c, n * sizeof(float), p.src, n * sizeof(float)) && !overlap(c, n * sizeof(float), p.src2, n * sizeof(float)) && (p.kind == 4 || (sca == p.sa && scb == p.sb))) {
             // the delta of a recorded ReLU backward pass copied into another zero delta: it joins the record
             int status = 0;
             if (lz_take(cx, st, c, n * sizeof(float), &status)) {

@@ -157,6 +157,39 @@ def test_relu_backward_with_copies(lib):
         L.call("set_option", b"lazy_zero", 0)
 
 
+@pytest.mark.parametrize("which", ["d", "act"])
+@pytest.mark.parametrize("shape", [(64, 4, 28, 28), (8, 2, 256, 256)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("then", ["bn_bwd", "axpby"])
+def test_relu_backward_whose_input_lies_in_the_next_output(lib, which, shape, then):
+    """relu_bwd reads d and act when it is called: what follows may write into their memory, half of which is part of its output here."""
+    L = lib
+    n, z, h, w = shape
+    rng = np.random.default_rng(8)
+    x, v, o = (rng.standard_normal(shape).astype(F) for _ in range(3))
+    g, b = rng.uniform(0.5, 1.5, z).astype(F), rng.standard_normal(z).astype(F)
+    E = x.size
+
+    def run(lazy):
+        L.call("set_option", b"lazy_zero", lazy)
+        try:
+            y, opa, r, gm, gv, me, va, dg, db = _forward(L, x, g, b)
+            gg, gb, m1, m2, dd, other = L.zeros((z,)), L.zeros((z,)), L.empty((z,)), L.empty((z,)), L.empty(shape), L.to_device(o)
+            arena = L.empty((E + E // 2,))
+            low, high = arena.addr, arena.addr + 4 * (E // 2)        # the output; the input that reaches into it
+            L.call("memcpy_h2d", 0, high, v.ctypes.data_as(ctypes.c_void_p), v.nbytes)
+            L.call("fill", 0, dd, E, 5.0); L.call("fill", 0, dd, E, 0.0); L.call("fill", 0, low, E, 0.0)
+            L.call("relu_bwd", 0, high if which == "d" else other, high if which == "act" else other, dd, E)
+            if then == "bn_bwd":
+                L.call("bn_bwd", 0, n, z, h * w, dd, opa, low, gg, gb, dg, va, m1, m2)
+            else:
+                L.call("axpby", 0, 1.0, dd, 1.0, low, low, 0, E)
+            return [t.numpy() for t in (dd, arena, gg, gb)]
+        finally:
+            L.call("set_option", b"lazy_zero", 0)
+    for got, want in zip(run(1), run(0)):
+        np.testing.assert_array_equal(got, want)
+
+
 def test_quotients_are_the_ieee_ones(lib):
     """Dividends of every magnitude (denormals, zeros, infinities and NaNs among them) by divisors with awkward mantissas: inference-mode
     BatchNorm with mean 0 computes x / sqrt(v + eps) per element."""
