@@ -23,6 +23,7 @@ int conv_tc_fwd(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, 
 // instead of added; routes that cannot use this write the zeros first.
 int conv_tc_bwd_data(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *dy, const float *w, float *dx, int precision, bool dx_zero);
 int conv_tc_gemm(DevCtx *cx, cudaStream_t st, const float *a, int ta, const float *b, int tb, float *c, int inc_c, int m, int n, int k, int precision);
+double conv_tc_gemm_us(int m, int n, int k);          // estimate of that product's time without its fixed costs
 bool conv_tc_allowed();          // false while eddlb200_set_option("conv_path", 1) / EDDL_B200_CONV=simt forces the fp32 FMA kernels
 int conv_tc_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const float *x, const float *dy, float *gw, int precision, bool gw_zero);
 

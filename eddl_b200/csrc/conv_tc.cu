@@ -2161,6 +2161,11 @@ int conv_tc_bwd_weight(DevCtx *cx, cudaStream_t st, const ConvGeom &g, const flo
     return run(cx, st, dev, 2, g, x, dy, gw, nullptr, precision, gw_zero);
 }
 
+double conv_tc_gemm_us(int m, int n, int k) {
+    const int bn = tile_n(n), kblocks = (k + BK - 1) / BK;
+    return pick_splits((long long)((m + BM - 1) / BM) * ((n + bn - 1) / bn), kblocks, gather_us(bn), (size_t)m * n, (kblocks + kMaxChainBlocks - 1) / kMaxChainBlocks).us;
+}
+
 // C[m x n] (row-major) = op(A) op(B), += when inc_c == 1, written into known zeros when inc_c == 2: the dense layers' GEMMs
 // (Tensor::mult2D, src/tensor/tensor_math.cpp) on the same kernel, as a "convolution" whose rows are the rows of op(A).
 // kNotTaken = the caller runs the fp32 FMA GEMM.

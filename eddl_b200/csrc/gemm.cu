@@ -3,8 +3,9 @@
 // gpu_sum2D_rowwise (gpu_math.cu:517-528) and gpu_reduce_sum2D (gpu_reduction.cu:232-244,
 // one atomicAdd per element); arithmetic as cpu_mult2D / cpu_sum2D_rowwise /
 // cpu_reduce_sum2D (src/hardware/cpu/cpu_math.cpp:302-325,369-380; cpu_reduction.cpp:91-112).
-// The dense layers of the nets are small (64 x 2048 x 1000), so this is an fp32 FMA
-// kernel; see sgemm_kernel.
+// Three kernels share the products, each where it is the fastest (pick_route): fp32 FMA with the k slices of a tile
+// meeting in cluster memory (sgemm_kernel), fp32 FMA with any number of k slices
+// meeting in memory (sgemm_split_kernel), and the convolutions' tensor-core kernel.
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "conv_common.cuh"
@@ -22,7 +23,8 @@ constexpr int kMaxCluster = 8;          // portable cluster size: k slices of on
 // with its own slice of k; the partial tiles meet in the blocks' shared memory, and every block adds its share of the rows from
 // all of them in slice order and stores it -- one launch, no partial sums in memory.  A k step of 32 is fetched into registers
 // while the one before it is multiplied (16-byte loads where VEC: rows and pointers 16-byte aligned), 4 x 4 outputs per
-// thread.  100 x 1024 x 1024: 30 us (tensor-core kernel with split-K and operand packing) -> 8 us; exact fp32.
+// thread.  A k step takes 2.45 us however few blocks there are (it is a chain of latencies): 100 x 1024 x 1024 is four of them, 13 us
+// against 22 on the tensor-core kernel with its split-K and operand packing; exact fp32.
 template <bool TA, bool TB_, bool VEC>
 __global__ void __launch_bounds__(TB) sgemm_kernel(const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C, int inc_c,
                                                    int m, int n, int k, int k_per_slice) {
@@ -126,6 +128,136 @@ int launch_sgemm(DevCtx *cx, cudaStream_t st, const float *a, const float *b, fl
     return 0;
 }
 
+// The same tile with any number of k slices, which leave partial tiles in memory (part; null = one slice, straight into C).  For
+// reductions that eight slices do not make short (8 x 2 x 100000: 70 us, 615 with eight), and, with half the step, for
+// outer products of up to 16 terms, where sgemm_kernel's step of 32 is mostly padding (4096 x 4096 x 1: 45 us against 60).
+constexpr int SBK = 16;
+__global__ void __launch_bounds__(TB) sgemm_split_kernel(const float *__restrict__ A, int ta, const float *__restrict__ B, int tb,
+                                                         float *__restrict__ C, int inc_c, int m, int n, int k, int k_per_split,
+                                                         float *__restrict__ part) {
+    EB_GRID_WAIT();
+    __shared__ float As[SBK][BM + 4];
+    __shared__ float Bs[SBK][BN + 4];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float acc[4][4] = {};
+    const int kbeg = blockIdx.z * k_per_split;
+    int kend = k;
+    if (part) { kend = min(k, kbeg + k_per_split); C = part + (size_t)blockIdx.z * m * n; inc_c = 0; }
+    for (int k0 = kbeg; k0 < kend; k0 += SBK) {
+        for (int e = threadIdx.x; e < BM * SBK; e += TB) {
+            // choose the traversal that is contiguous in memory
+            int mi, ki;
+            if (ta) { mi = e % BM; ki = e / BM; } else { ki = e % SBK; mi = e / SBK; }
+            const int gm = m0 + mi, gk = k0 + ki;
+            float v = 0.f;
+            if (gm < m && gk < kend) v = ta ? A[(size_t)gk * m + gm] : A[(size_t)gm * k + gk];
+            As[ki][mi] = v;
+        }
+        for (int e = threadIdx.x; e < BN * SBK; e += TB) {
+            int ni, ki;
+            if (tb) { ki = e % SBK; ni = e / SBK; } else { ni = e % BN; ki = e / BN; }
+            const int gn = n0 + ni, gk = k0 + ki;
+            float v = 0.f;
+            if (gn < n && gk < kend) v = tb ? B[(size_t)gn * k + gk] : B[(size_t)gk * n + gn];
+            Bs[ki][ni] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < SBK; kk++) {
+            float a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = As[kk][ty * 4 + i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx * 4 + j];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int gm = m0 + ty * 4 + i;
+        if (gm >= m) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int gn = n0 + tx * 4 + j;
+            if (gn >= n) continue;
+            float *c = C + (size_t)gm * n + gn;
+            *c = inc_c == 1 ? __fadd_rn(*c, acc[i][j]) : (inc_c == 2 ? __fadd_rn(0.f, acc[i][j]) : acc[i][j]);     // 2: c is known to hold zeros
+        }
+    }
+}
+
+// c[i] = (inc_c ? c[i] : 0) + part[0][i] + part[1][i] + ...   (fixed order)
+__global__ void __launch_bounds__(256) sgemm_combine_kernel(const float *__restrict__ part, float *__restrict__ c, size_t count, int splits, int inc_c) {
+    EB_GRID_WAIT();
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+        float v = inc_c ? c[i] : 0.f;
+        for (int z = 0; z < splits; z++) v = __fadd_rn(v, part[(size_t)z * count + i]);
+        c[i] = v;
+    }
+}
+
+int launch_split(DevCtx *cx, cudaStream_t st, const float *a, int ta, const float *b, int tb, float *c, int inc_c, int m, int n, int k, int splits, int kps) {
+    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM, splits);
+    const size_t count = (size_t)m * n;
+    float *part = splits > 1 ? (float *)scratch(cx, count * splits * sizeof(float)) : nullptr;
+    if (!part) grid.z = splits = 1, kps = k;               // no room for partial tiles: unsplit, straight into C
+    eb::launch(sgemm_split_kernel, grid, TB, 0, st, a, ta, b, tb, c, inc_c, m, n, k, kps, part);
+    EB_LAUNCH_CHECK("gpu_mult2D");
+    if (splits == 1) return 0;
+    eb::launch(sgemm_combine_kernel, grid_for(count, 256), 256, 0, st, part, c, count, splits, inc_c == 1);
+    EB_LAUNCH_CHECK("gpu_mult2D(combine)");
+    return 0;
+}
+
+// Which kernel runs a product.  The estimates (microseconds) are fits to 420 products of m, n and k between 1 and 100000, plain and
+// transposed, warm and with a flushed L2; over these the choice takes 10.9 ms where the best kernel for each would take 10.8,
+// the cluster kernel alone 19.6 and the other two alone 14.0.
+enum class Route { Cluster, Split, TensorCore };
+struct GemmPlan { Route route; int slices, kps; };
+GemmPlan pick_route(int m, int n, int k, bool ta, bool tc_allowed) {
+    const double mnk = (double)m * n * k;
+    const long long tiles = (long long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
+    // cluster kernel: two blocks per SM where the tiles alone do not give them, slices of at least 64 (two k steps)
+    int slices = 1;
+    while (slices < kMaxCluster && tiles * slices * 2 <= 2 * EDDLB200_NUM_SMS && k >= slices * 2 * 64) slices *= 2;
+    const int kps = ((k + slices - 1) / slices + BK - 1) / BK * BK, steps = kps / BK;
+    const GemmPlan cluster{Route::Cluster, slices, kps};
+    // split kernel: as many slices of at least 64 as give two blocks per SM
+    int splits = 1;
+    if (tiles < EDDLB200_NUM_SMS) {
+        splits = (int)((2 * EDDLB200_NUM_SMS + tiles - 1) / tiles);
+        if (splits > k / 64) splits = k / 64;
+        if (splits < 1) splits = 1;
+    }
+    const int skps = splits == 1 ? k : ((k + splits - 1) / splits + SBK - 1) / SBK * SBK;
+    if (splits > 1) splits = (k + skps - 1) / skps;
+    const GemmPlan split{Route::Split, splits, skps};
+    const bool tc = tc_allowed && k >= 32 && mnk >= 67108864.0;
+    // From 2^29 multiply-adds on (whatever the shape) the tensor cores win.
+    if (tc && mnk >= 536870912.0) return GemmPlan{Route::TensorCore, 1, k};
+    // Outer products: the stores count once there is more than a wave of tiles, the launch and the latency before that.
+    if (k <= SBK) return tiles <= 2 * EDDLB200_NUM_SMS ? cluster : split;
+    if (steps <= 4) return cluster;
+    const double waves = (double)tiles * slices / EDDLB200_NUM_SMS, cluster_us = 2.5 + steps * (1.3 * waves > 2.45 ? 1.3 * waves : 2.45);
+    double other_us;
+    if (tc) {
+        // the packing and the gather of a row-major A (not transposed: lanes run along m) grow with the rows of the first 128-row tile
+        const double rows = (m < 128 ? m : 128) / 128.0;
+        other_us = conv_tc_gemm_us(m, n, k) + (ta ? 10.0 * rows : 3.0 + 14.0 * rows) + 8.0 * m * (double)n / 5.0e6;
+    } else {
+        const double over = (double)tiles * splits / (2 * EDDLB200_NUM_SMS);
+        other_us = 5.0 + 2.65 * ((skps + SBK - 1) / SBK) * (over > 1.0 ? over : 1.0) + (splits > 1 ? 3.0 + 0.07 * splits : 0.0);
+    }
+    if (cluster_us <= 1.1 * other_us) return cluster;
+    return tc ? GemmPlan{Route::TensorCore, 1, k} : split;
+}
+
 __global__ void __launch_bounds__(256) rowbias_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ c, size_t total, int cols) {
     EB_GRID_WAIT();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -180,19 +312,14 @@ int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, flo
     }
     if (inc_c == 1) EB_MODIFIES(c, (size_t)m * n * sizeof(float)); else EB_WRITES(c, (size_t)m * n * sizeof(float));
     ProfScope prof(cx, PROF_GEMM, 2.0 * m * (double)n * k);
-    // Products of 2^29 multiply-adds or more run on the tensor-core kernel (3xTF32, like the convolutions).  Below that its fixed cost
-    // -- packing an operand, index tables, the split-K combine -- is more than the FMA kernel takes for the whole product
-    // (64 x 1000 x 2048 for ResNet-50's classifier: 29 -> 11 us), and a library forced to the FMA path stays here.
-    if (conv_tc_allowed() && k >= 32 && (double)m * n * k >= 536870912.0) {
+    GemmPlan plan = pick_route(m, n, k, ta != 0, conv_tc_allowed());          // a library forced to the FMA path stays on the FMA kernels
+    if (plan.route == Route::TensorCore) {
         const int r = conv_tc_gemm(cx, st, a, ta, b, tb, c, inc_c, m, n, k, 0);
         if (r != kNotTaken) return r;
+        plan = pick_route(m, n, k, ta != 0, false);
     }
-    // k slices: two blocks per SM where the tiles alone do not give them, slices of at least 64 (two k steps)
-    const long long tiles = (long long)((n + BN - 1) / BN) * ((m + BM - 1) / BM);
-    int slices = 1;
-    while (slices < kMaxCluster && tiles * slices * 2 <= 2 * EDDLB200_NUM_SMS && k >= slices * 2 * 64) slices *= 2;
-    int kps = (k + slices - 1) / slices;
-    kps = (kps + BK - 1) / BK * BK;
+    if (plan.route == Route::Split) return launch_split(cx, st, a, ta, b, tb, c, inc_c, m, n, k, plan.slices, plan.kps);
+    const int slices = plan.slices, kps = plan.kps;
     const bool vec = aligned16(a) && aligned16(b) && (ta ? m : k) % 4 == 0 && (tb ? k : n) % 4 == 0;
     if (ta) {
         if (tb) return vec ? launch_sgemm<true, true, true>(cx, st, a, b, c, inc_c, m, n, k, slices, kps) : launch_sgemm<true, true, false>(cx, st, a, b, c, inc_c, m, n, k, slices, kps);

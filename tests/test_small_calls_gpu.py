@@ -27,6 +27,39 @@ def test_mult2d_tiles_and_slices(lib, m, n, k, ta, tb, inc):
     assert np.all(np.abs(dc.numpy() - want) <= bound)
 
 
+# both sides of the lines between the kernels: outer products of up to 16 terms over few and many tiles, k steps of a slice, few and many
+# slices in memory, the tensor-core kernel from 2^26 multiply-adds on
+@pytest.mark.parametrize("m,n,k", [(1100, 1000, 16), (1200, 1600, 16), (1200, 1600, 17), (1200, 1601, 1), (1, 2, 4097), (3, 2, 30001), (1, 64, 12544), (65, 10, 4096), (5, 520, 8200),
+                                   (32, 1000, 1025), (8, 4096, 2100), (300, 1000, 1000), (64, 1000, 2048), (9600, 64, 70)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("inc", [0, 1])
+def test_mult2d_routes(lib, m, n, k, ta, tb, inc):
+    test_mult2d_tiles_and_slices(lib, m, n, k, ta, tb, inc)
+
+
+def _us(lib, fn, reps=20):
+    fn(); fn()
+    best = 1e9
+    for _ in range(3):
+        lib.call("timer_start", 0, 3)
+        for _ in range(reps):
+            fn()
+        lib.call("timer_stop", 0, 3)
+        ms = ctypes.c_float()
+        lib.call("timer_elapsed_ms", 0, 3, ctypes.byref(ms))
+        best = min(best, ms.value * 1e3 / reps)
+    return best
+
+
+def test_a_long_reduction_is_spread_over_the_gpu(lib):
+    """8 x 2 outputs: with an eighth of the reduction a call is bound by its launches, so eight times as many terms must cost less than five
+    times as much (a fixed number of slices: eight times; measured 70 against 25 us)."""
+    def us(k):
+        a, b, c = lib.zeros((8, k)), lib.zeros((k, 2)), lib.empty((8, 2))
+        return _us(lib, lambda: lib.call("mult2d", 0, a, 0, b, 0, c, 0, 8, 2, k))
+    assert us(100000) < 5 * us(12500)
+
+
 @pytest.mark.parametrize("shape", [(2, 3, 2, 2), (3, 5, 28, 28), (2, 4, 7, 7), (1, 2, 9, 12), (2, 2, 12, 10), (1, 3, 5, 6)])
 @pytest.mark.parametrize("lazy", [0, 1])
 def test_maxpool_2x2_stride_2(lib, shape, lazy):
