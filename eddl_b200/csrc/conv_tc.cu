@@ -1562,8 +1562,14 @@ double gather_layer_us(const ConvGeom &g, int mode) {
 
 // What the row-shift kernel would do with a layer: the padded position space, slabs and classes (see conv_rs.cuh), tile width and
 // number of splits.  false = the layer does not fit it.
-struct RsPlan { RsParams P; int bn, smem, kblocks; double us; };
-bool conv_rs_plan(const ConvGeom &g, int mode, int precision, RsPlan &plan) {
+struct RsPlan { RsParams P; int bn, smem, kblocks; double us, strided_us; };
+// A dx of which not every pixel is written costs whole sectors, after a fill where zeros are owed.
+double strided_dx_us(const ConvGeom &g, int classes, bool accumulate) {
+    if (classes >= std::min(g.sr, g.ih) * std::min(g.sc, g.iw)) return 0.0;
+    const double rows_us = 4.0 * g.n * (double)g.c * ((g.ih + g.sr - 1) / g.sr) * g.iw / 5.0e6;
+    return accumulate ? 2.0 * rows_us : 4.0 * g.n * (double)g.c * g.ih * g.iw / 5.0e6 + 0.5 * rows_us;
+}
+bool conv_rs_plan(const ConvGeom &g, int mode, int precision, bool accumulate, RsPlan &plan) {
     RsParams &P = plan.P;
     P = RsParams{};
     const int planes = precision == 1 ? 1 : 2;
@@ -1666,6 +1672,22 @@ bool conv_rs_plan(const ConvGeom &g, int mode, int precision, RsPlan &plan) {
     plan.smem = 1024 + P.nbuf * planes * P.slab_plane + P.bst * stage + RS_BAR_WORDS * 8 + 64;
     const int chain = ((max_kb + P.splits - 1) / P.splits) * (std::min(P.C, BK) + 7) / 8;
     P.nmain = chain > 64 ? NMAIN : 1;
+    // What the chosen tiling takes, for the choice of the kernel.  Beyond the estimate above: a K-block waits for its weights when the ring
+    // is short (a copy takes 1.05 us); the second pass over a slab's rows runs beside the first, later ones wait for their loads
+    // (longer where a tile has a single slab); an accumulating epilogue takes 9 us per tile (reads of the old values, eight at a
+    // time), hidden only behind as much work.  Fitted to 364 layers of one to 64 images in three passes: without these terms, and
+    // with the single-CTA kernels' strided dx taken as twice a dense one, 29 of 1092 went to this kernel although another was up
+    // to 1.5 times as fast (35 x 832 x 21 x 69, 16 filters, 3 x 3, into a dx that holds values: 188 us against 127), now three, by 5 us at
+    // most; all of them together take 61.0 ms, 61.7 before, 60.4 with the best kernel for each.
+    const int c_i = plan.bn == 32 ? 0 : plan.bn == 64 ? 1 : 2, passes = (rows + 127) / 128;
+    const double kb_us = std::max(c_kb[c_i], 1.05 / P.bst), pass_us = (1.1 * passes + (P.cgs == 1 ? 2.2 : 1.1) * std::max(passes - 2, 0)) * (P.ssc > 1 ? 1.8 : 1.0);
+    const long long items = (long long)P.tiles_m * P.tiles_n, rounds = (items * P.ncls * P.splits + 73) / 74;
+    double group = 0;
+    for (int q = 0; q < nslab; q++) group += std::max(P.slab[q].ntaps * kb_us, pass_us);
+    plan.us = 4.0 + (double)rounds / P.ncls * (std::max(group * P.cgs / P.splits, pass_us) + (c_i == 2 ? 2.6 : 1.3) * P.ncls);
+    if (P.splits > 1) plan.us += 4.5 + (double)items * P.ncls * P.splits * plan.bn * 256 * 8 / 5.0e6;
+    else if (accumulate) plan.us += (double)(rounds - 1) * std::max(0.0, 9.0 - (plan.us - 4.0) / rounds) + 4.0;
+    plan.us += plan.strided_us = mode == 1 ? strided_dx_us(g, P.ncls, accumulate) : 0.0;
     return true;
 }
 
@@ -1676,15 +1698,19 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
            int precision, bool out_zero) {
     if (!g_conv_rs) return kNotTaken;
     RsPlan plan;
-    if (!conv_rs_plan(g, mode, precision, plan)) return kNotTaken;
+    if (!conv_rs_plan(g, mode, precision, mode == 1 && !out_zero, plan)) return kNotTaken;
     RsParams &P = plan.P;
     if (g_conv_rs < 2) {
         // Layers of a few channels stay on the gather kernels (a K-block here is 32 channels of one tap), layers of a few dx channels
         // with their GEMM route; otherwise the smaller estimate wins.
         if (P.C < 16 || P.K < 8 || (mode == 1 && g.c <= 8)) return kNotTaken;
         const bool dense = g.sr == 1 && g.sc == 1;
-        double other = gather_layer_us(g, mode);
-        if (mode == 1 && !dense) other *= 2.0;                            // one launch per parity class, none of them split
+        double other = dense || mode == 0 ? gather_layer_us(g, mode) : plan.strided_us + (P.ncls > 1 ? 8.0 * g.n * (double)g.c * g.ih * g.iw / 5.0e6 : 0.0);
+        for (int c = 0; c < P.ncls && !dense && mode == 1; c++) {             // one launch per parity class, none of them split, sectors of dx shared by two
+            const int bn = tile_n(P.K);
+            const long long tiles = ((long long)g.n * P.cls[c].dh * P.cls[c].dw + BM - 1) / BM * ((P.K + bn - 1) / bn);
+            other += 8.0 + (double)((tiles + EDDLB200_NUM_SMS - 1) / EDDLB200_NUM_SMS) * ((P.C * P.cls[c].taps + BK - 1) / BK * gather_us(bn) + 3.0);
+        }
         const int bn = tile_n(P.K), tiles_n = (P.K + bn - 1) / bn, pq = g.oh * g.ow;
         if (g.kr == 1 && g.kc == 1 && g.pt == 0 && g.pl == 0 && P.C >= 32 && P.K >= 32 && pq >= 32)
             other = std::min(other, tma_fed_us(((long long)g.n * ((pq + 31) / 32) + 3) / 4 * tiles_n, P.cgs) +
@@ -1692,7 +1718,7 @@ int run_rs(DevCtx *cx, cudaStream_t st, int dev, int mode, const ConvGeom &g, co
                                         (dense ? 0.0 : 6.0 + 8.0 * g.n * (mode == 0 ? g.c : g.c * g.sr * g.sc) * (double)pq / 5.0e6));
         if (dense && g.kr == 3 && g.kc == 3 && g.pt == 1 && g.pl == 1 && g.iw == g.ow && g.ih == g.oh && pq % 4 == 0 && pq >= 64 && g.iw <= 61 && P.C >= 32 && P.K >= 32)
             other = std::min(other, tma_fed_us((long long)g.n * ((pq + BM - 1) / BM) * tiles_n, 9 * P.cgs));
-        if (plan.us > 0.95 * other) return kNotTaken;
+        if (plan.us > other - 0.8) return kNotTaken;
     }
     const int planes = precision == 1 ? 1 : 2;
     if (mode == 1 && out_zero) {

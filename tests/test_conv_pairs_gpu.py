@@ -1,6 +1,8 @@
 """GPU parity of the row-shift convolution on CTA pairs ("conv_pairs" 2 = wherever it fits), forward and backward-data, at the edges of
 its tiles, slabs and classes: one position more or less than a tile, filters that leave the image on every side, partly filled
 channel groups and filter tiles, both strides, splits of the reduction, accumulation into dx."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -80,3 +82,40 @@ def test_repeated_calls_give_the_same_bits(pairs):
         for _ in range(3):
             L.call("conv2d_fwd", 0, x, wt, None, y, *geo)
             np.testing.assert_array_equal(y.numpy(), first)
+
+
+# n, c, h, w, k, kernel, stride, pad, precision, pass: short reductions into a dx that holds values, slabs of several passes, two weight
+# stages, a dx of which every fourth pixel is written
+SLOWER_ON_PAIRS = [(35, 832, 21, 69, 16, 3, 1, 1, 2, "bwd_data"), (34, 704, 20, 49, 16, 3, 1, 0, 0, "bwd_data"), (31, 48, 18, 72, 247, 5, 1, 2, 0, "bwd_data"),
+                   (27, 16, 70, 70, 208, 3, 1, 0, 2, "fwd"), (64, 256, 56, 56, 512, 1, 2, 0, 0, "bwd_data")]
+
+
+@pytest.mark.parametrize("case", SLOWER_ON_PAIRS, ids=lambda c: "-".join(map(str, c)))
+def test_layers_that_pairs_would_slow_down_stay_on_the_other_kernels(lib, case):
+    """The default choice against the same call with CTA pairs off: these layers took 1.13 to 1.5 times as long on pairs (the bound leaves
+    room for the spread of single launches, a few percent)."""
+    L = lib
+    n, c, h, w, k, r, s, p, precision, which = case
+    oh, ow = (h + 2 * p - r) // s + 1, (w + 2 * p - r) // s + 1
+    x, y, wt = L.zeros((n, c, h, w)), L.zeros((n, k, oh, ow)), L.zeros((k, c, r, r))
+    geo = (n, c, h, w, k, r, r, oh, ow, s, s, p, p, precision)
+
+    def us(pairs):
+        L.call("set_option", b"conv_pairs", pairs)
+        times = []
+        for _ in range(25):
+            L.call("timer_start", 0, 3)
+            if which == "fwd":
+                L.call("conv2d_fwd", 0, x, wt, None, y, *geo)
+            else:
+                L.call("conv2d_bwd_data", 0, y, wt, x, *geo)
+            L.call("timer_stop", 0, 3)
+            ms = ctypes.c_float()
+            L.call("timer_elapsed_ms", 0, 3, ctypes.byref(ms))
+            times.append(ms.value * 1e3)
+        return float(np.median(times[5:]))
+    try:
+        off, default = us(0), us(1)
+    finally:
+        L.call("set_option", b"conv_pairs", 1)
+    assert default <= 1.08 * off + 2
