@@ -328,11 +328,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WG_THREADS, 1) conv_
                         float *q = p;
 #pragma unroll
                         for (int j = 0; j < 32; j++) { *q = __fadd_rn(0.f, acc[c][j]); q += step; }
+                    } else if (P.accumulate) {
+                        // eight old values at a time: a load cannot be moved above the store before it, and one by one the 64 round
+                        // trips of a row are longer than the reduction of a small layer (48 x 720 channels, 10 x 8, one image: 41 us)
+#pragma unroll
+                        for (int h = 0; h < 32; h += 8) {
+                            float prev[8];
+#pragma unroll
+                            for (int j = 0; j < 8; j++) prev[j] = h + j < ncols ? __ldcg(p + (h + j) * step) : 0.f;
+#pragma unroll
+                            for (int j = 0; j < 8; j++) if (h + j < ncols) p[(h + j) * step] = __fadd_rn(prev[j], acc[c][h + j]);
+                        }
                     } else {
                         float *q = p;
 #pragma unroll
                         for (int j = 0; j < 32; j++)
-                            if (j < ncols) { *q = P.accumulate ? __fadd_rn(__ldcg(q), acc[c][j]) : __fadd_rn(0.f, acc[c][j]); q += step; }
+                            if (j < ncols) { *q = __fadd_rn(0.f, acc[c][j]); q += step; }
                     }
                     p += 32 * step;
                 }

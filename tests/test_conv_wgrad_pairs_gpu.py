@@ -1,6 +1,8 @@
 """GPU parity of backward-weight on CTA pairs ("conv_pairs" 2 = wherever it fits) at the edges of its tiles: one channel or filter more
 or less than a tile, a second CTA with nothing to do, planes that end inside a K-block, the widest slab, split and unsplit
 reductions, accumulation into the gradient and the store into known zeros."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -51,3 +53,30 @@ def test_backward_weight(pairs, case, precision, limit, zero):
         L.call("sync", 0)
     finally:
         L.call("set_option", b"lazy_zero", 0)
+
+
+@pytest.mark.parametrize("case", [(1, 48, 10, 8, 720), (2, 16, 7, 8, 592)], ids=lambda c: "-".join(map(str, c)))
+def test_accumulating_into_the_gradient_of_a_small_layer_is_not_slower_on_pairs(lib, case):
+    """A reduction of a few K-blocks, so that adding to the gradient is most of the call: the default choice against the same call with
+    CTA pairs off (1.8 times as long with one old value in flight per thread)."""
+    L = lib
+    n, c, h, w, k = case
+    x, dy, gw = L.zeros((n, c, h, w)), L.zeros((n, k, h, w)), L.zeros((k, c, 3, 3))
+    geo = (n, c, h, w, k, 3, 3, h, w, 1, 1, 1, 1, 0)
+
+    def us(pairs):
+        L.call("set_option", b"conv_pairs", pairs)
+        times = []
+        for _ in range(25):
+            L.call("timer_start", 0, 3)
+            L.call("conv2d_bwd_weight", 0, x, dy, gw, None, *geo)
+            L.call("timer_stop", 0, 3)
+            ms = ctypes.c_float()
+            L.call("timer_elapsed_ms", 0, 3, ctypes.byref(ms))
+            times.append(ms.value * 1e3)
+        return float(np.median(times[5:]))
+    try:
+        off, default = us(0), us(1)
+    finally:
+        L.call("set_option", b"conv_pairs", 1)
+    assert default <= 1.2 * off + 2
