@@ -633,6 +633,16 @@ inline unsigned pick_split(unsigned z, unsigned per_channel) {
     return s;
 }
 
+// Whether a ReLU backward pass is folded in: not where the two-pass kernels go element by element (planes that are no multiple of
+// four long, unaligned tensors).  Every element then costs three or four 4-byte loads in each pass, and the separate ReLU pass,
+// which does not care about planes, is the cheaper one: 64 x 64 x 27 x 27 48 us folded, 36 separate.  Short planes in many
+// channels of one slice are the exception (64 x 1024 x 7 x 7 28 and 32).  With 16-byte loads 64 x 512 x 28 x 28 takes 111 to 140 us
+// folded, 155 separate.
+bool fold_pays(unsigned z, unsigned per, unsigned rc, int tensors, bool vec) {
+    OnePlan p;
+    return vec || one_plan(z, per, rc, tensors, vec, p) || (rc < 64 && z >= 512 && pick_split(z, per) == 1);
+}
+
 }  // namespace
 
 namespace eb {
@@ -705,11 +715,13 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
             const size_t tb = elements * sizeof(float), zb = (size_t)z * sizeof(float);
             apart = apart && !overlap(in, tb, pdelta, tb) && !overlap(in, tb, gbn_g, zb) && !overlap(in, tb, gbn_b, zb) && !overlap(in, tb, mean1, zb) && !overlap(in, tb, mean2, zb);
         }
-        if (p.kind == 4 && p.dst == delta && p.n == elements && apart) {
+        const float *own = nullptr;                                      // beta, where what ReLU tests can be computed again
+        if (p.kind == 4 && p.dst == delta && p.n == elements && apart) own = bn_g ? bn_source_beta(cx, p.src2, opa, bn_g, elements, z, rc) : nullptr;
+        if (p.kind == 4 && p.dst == delta && p.n == elements && apart &&
+            fold_pays(z, (unsigned)b * rc, rc, own ? 2 : 3, rc % 4 == 0 && aligned16(delta) && aligned16(opa) && aligned16(pdelta) && aligned16(p.src) && (own || aligned16(p.src2)))) {
             // the ReLU backward pass that makes this delta is still on record: it is folded in
             p.active = false;
-            src = p.src; act = p.src2;
-            beta = bn_g ? bn_source_beta(cx, act, opa, bn_g, elements, z, rc) : nullptr;
+            src = p.src; act = p.src2; beta = own;
             mask = beta ? 2 : 1;
         } else if (int r = pend_copy_flush(cx, st)) return r;
     }

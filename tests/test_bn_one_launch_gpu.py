@@ -133,6 +133,38 @@ def test_relu_backward_folded_in_under_another_layout(lib, layout):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("shape,folds", [((27, 53, 37, 41), False), ((6, 1866, 79, 11), False), ((125, 296, 2, 29), False), ((64, 1024, 7, 7), True), ((128, 512, 7, 7), True), ((8, 200, 25, 25), True), ((64, 64, 28, 28), True)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else "")
+@pytest.mark.parametrize("own", [True, False])
+def test_relu_backward_is_folded_in_where_that_is_cheaper(lib, shape, folds, own):
+    """Scalar two-pass planes in slices, long ones in one slice, short ones with few and with many channels, planes of one launch, 16-byte planes."""
+    L = lib
+    n, z, h, w = shape
+    rng = np.random.default_rng(z)
+    x, d, other = (rng.standard_normal(shape, dtype=F) for _ in range(3))
+    g, b = rng.uniform(0.5, 1.5, z).astype(F), rng.standard_normal(z).astype(F)
+    E = x.size
+
+    def run(lazy):
+        L.call("set_option", b"lazy_zero", lazy)
+        try:
+            y, opa, r, gm, gv, me, va, dg, db = _forward(L, x, g, b)
+            act = y if own else L.to_device(other)
+            dd, pd, gg, gb, m1, m2 = L.empty(shape), L.empty(shape), L.zeros((z,)), L.zeros((z,)), L.empty((z,)), L.empty((z,))
+            for a in (dd, pd):
+                L.call("fill", 0, a, E, 0.0)
+            src, before = L.to_device(d), launches(L)
+            L.call("relu_bwd", 0, src, act, dd, E)
+            L.call("bn_bwd", 0, n, z, h * w, dd, opa, pd, gg, gb, dg, va, m1, m2)
+            return launches(L) - before, [t.numpy() for t in (dd, pd, gg, gb, m1, m2)]
+        finally:
+            L.call("set_option", b"lazy_zero", 0)
+    (launched, got), (separate, want) = run(1), run(0)
+    assert launched == separate - (1 if folds else 0)
+    for a, b in zip(got, want):
+        np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-5)
+
+
 def test_relu_backward_with_copies(lib):
     """relu_bwd whose result is added into one or two zero deltas next (LAdd): one kernel, the bits of the separate calls; and a
     record that nothing takes over is run by the next call."""
