@@ -38,9 +38,8 @@ __device__ __forceinline__ Slice slice_of(unsigned per_channel, unsigned nsplit,
     return r;
 }
 
-// Quotients by one divisor.  The reference divides every element by its channel's sigma, and the IEEE division that CUDA provides is
-// a reciprocal seed, its refinement and range checks per element -- a third of a BatchNorm kernel's instructions.  With the
-// correctly rounded reciprocal r of the divisor in hand, Markstein's method (P. Markstein, Computation of elementary functions on
+// Quotients by one divisor.  The reference divides every element by its channel's sigma, and an IEEE division per element is a third
+// of a BatchNorm kernel's instructions.  With the correctly rounded reciprocal r of the divisor in hand, Markstein's method (P. Markstein, Computation of elementary functions on
 // the IBM RISC System/6000 processor, 1990) gives the same correctly rounded quotient in five multiply-adds: q = a r, one
 // correction makes q faithful, a second one with the exact remainder rounds it correctly.  It needs every intermediate in
 // the normal range: dividends outside 2^-60 .. 2^60 (zeros, infinities and NaNs among them) and divisors outside 2^-30 .. 2^30 take
@@ -768,8 +767,8 @@ int eddlb200_bn_bwd(int dev, int b, int z, int rc, float *delta, const float *op
 // process whose device memory has been handed over in full to another allocator (a cudaMalloc
 // from a plug-in then fails or fragments that pool), or a latency-critical loop in which the
 // implicit device synchronisation of cudaMalloc / cudaFree is not acceptable.  For them this
-// entry point runs the same two kernels with the partial sums in a fixed array that is part of
-// the library image: kNoAllocPairs (sum, sum-of-squares) pairs = 2 MiB of device memory, held by
+// entry point runs the same kernels, small tensors in one launch without partial sums and the
+// others with the partial sums in a fixed array that is part of the library image: kNoAllocPairs (sum, sum-of-squares) pairs = 2 MiB of device memory, held by
 // every GPU that loads the library until the process exits.
 //
 // * It calls no cudaMalloc / cudaFree / cudaMallocHost and does not create the library's device

@@ -3,7 +3,7 @@
 // What bounds a 3xTF32 convolution on this GPU is not the tensor pipe but shared-memory bandwidth (128 bytes per SM and cycle).
 // For a 128 x 128 tile, a K-block of 32 costs 12 MMAs of 64 cycles; with one operand tile per filter tap and one CTA per tile
 // the same K-block moves 384 cycles' worth of bytes through the conversion of the activations (load, split, two stores), 768 through
-// the MMAs' operand reads and 256 through the copy of the weights: 1436 cycles, which is what such a kernel measures (1437).
+// the MMAs' operand reads and 256 through the copy of the weights: 1408 cycles by this count (not all of it in a row: about 1300 measured).
 // Here
 //   * the activations are converted ONCE per 32-channel group, not once per tap.  Pixels are numbered in a padded space: image
 //     rows of pitch Wp (the image width plus the larger of the two side paddings), images of Hp rows, the padding reading as
@@ -14,7 +14,9 @@
 //   * two CTAs of a cluster work on 256 positions x BN filters with M = 256 instructions: each holds its own 128 positions and HALF
 //     of the weights, which halves the traffic of the weight copies and a quarter of the operand reads.
 // Per K-block and SM: conversion 81 cycles (56 x 56 images), operand reads 576, weights 128 -- 785, just above the 768 of the
-// MMAs.  Measured, 64 x 256 x 56 x 56, 256 filters, 3 x 3: 1.12 -> 0.73 ms forward (run_rs has the rule for where it is used).
+// MMAs; measured 833 with fill and drain, the tensor pipe busy 92 % of the time (profiles/conv_pairs_bn_gemm.md).  64 x 256 x 56 x 56,
+// 256 filters, 3 x 3 forward, igemm_tc_kernel -> this kernel: single launches behind a flushed L2 1.04 -> 0.81 ms; back to back
+// for a second, where the power cap holds the SM clock at 1.53 GHz, 0.93 ms (run_rs has the rule for where it is used).
 //
 // Positions run across images, so planes of any size and width fill whole tiles (what is lost is the padding: 1 column per row and
 // 1 row per image), the halo is read with plain loads and the channel count need not be a multiple of anything.  Strides:

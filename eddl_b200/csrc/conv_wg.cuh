@@ -8,10 +8,12 @@
 //     operand reads of the MMAs       96 KB        72 KB         96 KB        72 KB
 //     cycles                          1536         1152          1616         1228
 // A pair computes 256 rows with M = 256 instructions; each CTA lands, converts and holds its own 128 rows of A and HALF of B.
-// Measured (whole call, 3xTF32, igemm_tc_kernel on the same layer -> this kernel): 64 x 256 x 56 x 56, 256 filters, 3x3: 1560 -> 1175 us;
-// 64 x 128 x 28 x 28, 3x3: 117 -> 84; 64 x 256 x 14 x 14, 3x3: 133 -> 95; 64 x 1024 x 14 x 14, 256 filters, 1x1: 46 -> 36;
-// 64 x 512 x 28 x 28, 256 filters, 1x1: 78 -> 62.  With one lane per pixel and 4-byte accesses in the SLAB producers the first of
-// these took 1516 us: four times the shared-memory instructions for the same bytes.
+// The counts are upper bounds; measured with fill and drain: 1172 cycles (3x3 pair, tensor pipe busy 65 %) and 1067 (1x1 pair, 70 %),
+// profiles/conv_pairs_bn_gemm.md.
+// Whole calls, single launches behind a flushed L2, 3xTF32, igemm_tc_kernel on the same layer -> this kernel: 64 x 256 x 56 x 56, 256
+// filters, 3x3: 1574 -> 1181 us; 64 x 128 x 28 x 28, 3x3: 126 -> 93; 64 x 256 x 14 x 14, 3x3: 142 -> 106; 64 x 1024 x 14 x 14, 256
+// filters, 1x1: 52 -> 44; 64 x 512 x 28 x 28, 256 filters, 1x1: 81 -> 67.  With one lane per pixel and 4-byte accesses in the SLAB
+// producers the first of these took 1516 us: four times the shared-memory instructions for the same bytes.
 //
 // SLAB = false, 1x1 stride-1 unpadded layers: A rows are the channels of x or, swapped, the filters of dy -- whichever fills 256
 // rows better -- and the landed values are the hi planes as they are.  SLAB = true, 3x3 stride-1 "same" layers: the 128 rows of a

@@ -511,7 +511,7 @@ static cudaEvent_t peer_event(cudaEvent_t &slot) {
 
 // Device code outside this library is about to write (or has written) [p, p + bytes): everything the library still owes
 // the range is written first (deferred zero fills, a pending copy, an average in flight), and whatever the library caches
-// about its contents (packed weight images, the loss / metric pair) is invalidated.
+// about its contents (packed weight images, the loss / metric pair, what a BatchNorm output was computed from) is invalidated.
 int eddlb200_notify_write(int dev, void *p, size_t bytes) {
     EB_CTX(dev);
     if (!p || !bytes) return 0;

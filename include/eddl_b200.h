@@ -49,7 +49,8 @@ int eddlb200_memcpy_d2d(int dev, void *dst, const void *src, size_t bytes);
 int eddlb200_memcpy_peer(int dst_dev, void *dst, int src_dev, const void *src, size_t bytes);
 /* For device code OUTSIDE this library that writes memory this library also works on: call it before enqueueing the write on
  * the library's stream (eddlb200_stream).  Zeros, copies and averages the library still owes the range are written first, and
- * what it caches about the range's contents (packed weight images of the convolutions, the loss / metric pair) is dropped.
+ * what it keeps about the range's contents (packed weight images of the convolutions, the loss / metric pair, what a BatchNorm
+ * output was computed from) is dropped.
  * The reference's host code never needs it: all its device writes are calls of this library. */
 int eddlb200_notify_write(int dev, void *p, size_t bytes);
 /* Pinned-host staged copies for a caller that overlaps transfers itself
@@ -231,9 +232,9 @@ int eddlb200_rand_binary(int dev, float *a, size_t n, float p, size_t seed, size
 /* ---- dense algebra (src/hardware/gpu/gpu_math.cu:457-528; gpu_reduction.cu:232-244;
  *      src/hardware/cpu/cpu_math.cpp:302-325,369-401) */
 /* gpu_mult2D: C[m,n] = (inc_c ? C : 0) + op(A) * op(B), row-major; A is [m,k] (or [k,m]
- * when ta), B is [k,n] (or [n,k] when tb).  Large products (k >= 32, m n k >= 2^26) run on the
- * tensor-core kernel of the convolutions in its fp32-equivalent 3xTF32 mode (about 1e-6 relative); smaller ones, and all of
- * them under "conv_path" 1, on an exact-fp32 FMA kernel. */
+ * when ta), B is [k,n] (or [n,k] when tb).  Large products (k >= 32, m n k >= 2^29, or from
+ * 2^26 on where it is the faster one) run on the tensor-core kernel of the convolutions in its fp32-equivalent 3xTF32 mode
+ * (about 1e-6 relative); the others, and all of them under "conv_path" 1, on exact-fp32 FMA kernels. */
 int eddlb200_mult2d(int dev, const float *a, int ta, const float *b, int tb, float *c, int inc_c,
                     int m, int n, int k);
 int eddlb200_sum2d_rowwise(int dev, const float *a, const float *b, float *c, int rows, int cols); /* C = A + b[col] */
@@ -254,9 +255,12 @@ int eddlb200_reduce_sum2d(int dev, const float *a, float *b, int rows, int cols,
  *          eddlb200_axpby(s, a, t, c, c, 0) into such a c is recorded and runs with the next call (fused with it when
  *          that is the second in-place add into c; the sum then stays on record for one more call and is fused
  *          with an eddlb200_relu_fwd of c); eddlb200_relu_bwd into such a pd is recorded in the same way and fused with an
- *          eddlb200_bn_bwd of pd or with adds of pd into other deltas that are owed zeros.  Off by default: device
- *          code outside this library does not see a deferred fill.  0 writes everything still deferred and returns
- *          to immediate fills.
+ *          eddlb200_bn_bwd of pd or with adds of pd into other deltas that are owed zeros: it READS d AND i IN THE NEXT CALL of
+ *          this library.  Where i is the output of an affine eddlb200_bn_fwd in training mode, eddlb200_bn_bwd computes i again
+ *          from opa, gamma and beta instead of reading it.  Off by default: device code outside this library does not see a
+ *          deferred fill or a recorded call.  While it is on, such code announces its writes to operands of recorded calls, to
+ *          buffers that are owed zeros and to a BatchNorm's output, opa, gamma and beta with eddlb200_notify_write BEFORE it
+ *          makes them.  0 writes everything still deferred and returns to immediate fills.
  *          "conv_prefetch" 1 (default) = in 1x1 unpadded layers a spare warp of the tensor-core kernel prefetches the
  *          activation operand into L2 ahead of the gather (results unchanged); 0 = off.
  *          "conv_tma" 2 (default) = forward and backward-data of 1x1 stride-1 unpadded layers (planes of a multiple of 4
@@ -264,8 +268,10 @@ int eddlb200_reduce_sum2d(int dev, const float *a, float *b, int rows, int cols,
           stores, or TMA fp32 adds where the output accumulates; 1 = only where the output is stored; 0 = the gather
           kernel everywhere.  Results are the same bits at every level.
  *          "conv_pairs" 1 (default) = forward and backward-data of layers with 16 channels or more run on pairs of CTAs that convert
- *          the activations once for all filter taps, where an estimate says that this is the faster kernel; 2 = wherever it fits;
- *          0 = never.  The reduction is ordered (channel group, tap, channel): agreement with the other kernels to rounding.
+ *          the activations once for all filter taps, and backward-weight of the 1x1 and 3x3 layers of "conv_tma_wgrad" and
+ *          "conv_tma_wgrad_3x3" on pairs that share an operand, where an estimate says that this is the faster kernel; 2 =
+ *          wherever it fits; 0 = never.  Forward and backward-data are reduced in the order (channel group, tap, channel):
+ *          agreement with the other kernels to rounding.
  *          "conv_tma_3x3" 1 (default) = forward and backward-data of 3x3 stride-1 pad-1 layers (planes of a multiple of 4
  *          pixels and at least 64, rows of at most 125 pixels, at least 32 channels on both sides) read raw slabs of the
  *          activations delivered by TMA, one per tile and 32-channel group for all nine taps; the reduction is then
